@@ -212,6 +212,31 @@ def test_tcgen05_one_and_two_issuers_agree(capi, m, k, n):
     assert float((d == 0).float().mean()) > 0.9
 
 
+@pytest.mark.parametrize("m,k,n,gs,asym,scale_dtype", [
+    (20, 14336, 136, 128, False, torch.float32),     # two tiles, sixteen CTAs each; last column tile eight wide
+    (17, 8256, 130, 64, True, torch.bfloat16),       # K = 32 x 256 + 64: void stage; group of 64; odd row pitch of the scales
+    (129, 14400, 132, 32, False, torch.bfloat16),    # two row tiles, groups of 32
+    (64, 12288, 257, 12288, True, torch.float32),    # one group, odd number of columns
+    (190, 16384, 128, 256, False, torch.float32)])   # one 192-token tile
+def test_tcgen05_shared_tiles(capi, m, k, n, gs, asym, scale_dtype):
+    """Few tiles with a long K: their chunks are dealt to many CTAs and the pieces added by the last to arrive.
+    Against the oracle; against the form in which one CTA sums a tile (bit 24; the two round one fp32 sum
+    differently, so one bf16 ulp); twice the same bits; with a post-op chain that reads two operands."""
+    x, q, s, z, b = make_woq_case(m, k, n, gs, seed=m + k, asym=asym, scale_dtype=scale_dtype)
+    y, packed = _run(capi, x, q, s, z, b, capi.ZT_ALGO_TCGEN05)
+    assert_close_bf16(y, O.woq_linear(x, packed.t(), s, z, b), what=f"shared tiles {m}x{k}x{n}")
+    again, _ = _run(capi, x, q, s, z, b, capi.ZT_ALGO_TCGEN05)
+    assert torch.equal(y, again)
+    one, _ = _run(capi, x, q, s, z, b, capi.ZT_ALGO_TCGEN05 | capi.ZT_ALGO_SINGLE_ISSUER)
+    d = (y.float() - one.float()).abs()
+    assert float((d - 2 ** -7 * y.float().abs()).max()) <= 1e-4 * float(y.float().abs().max())
+    ops, nbuf = POST_CASES["mul_add"]
+    g = torch.Generator().manual_seed(9)
+    bufs = [torch.randn(m, n, generator=g).to(torch.bfloat16) for _ in range(nbuf)]
+    ym, _ = _run(capi, x, q, s, z, b, capi.ZT_ALGO_TCGEN05, ops, bufs)
+    assert_close_bf16(ym, O.woq_linear(x, packed.t(), s, z, b, ops, bufs), what=f"shared tiles, mul_add {m}x{k}x{n}")
+
+
 @pytest.mark.parametrize("name", sorted(["relu", "gelu_erf", "silu", "add", "mul_add", "add_add"]))
 def test_tcgen05_post_ops(capi, name):
     ops, nbuf = POST_CASES[name]

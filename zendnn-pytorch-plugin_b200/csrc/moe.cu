@@ -14,7 +14,7 @@ namespace zt {
 
 namespace {
 
-constexpr int kRowTile = 64;  // token rows per GEMM tile (about the mean group size of the target config)
+constexpr int kRowTile = 128;  // token rows per GEMM tile: an expert's weights are converted once per row tile
 
 struct MoeLayout {
   size_t counts, offsets, cursor, tile_count, tiles, sorted_src, inv_pos, xs, h, a, o, total;
