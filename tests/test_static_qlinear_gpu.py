@@ -179,6 +179,17 @@ def test_argument_checks(capi):
                             c["ws"].cuda())
 
 
+@pytest.mark.parametrize("zp", [0, 255, -7, 300])          # the last two take the 64-bit correction
+@pytest.mark.parametrize("post", [(), (O.POST_SIGMOID,), (O.POST_MUL, O.POST_RELU, O.POST_ADD)])
+def test_zero_point_range_and_post_chains(capi, zp, post):
+    m, k, n = 130, 272, 131                                # ragged rows, columns and k-blocks
+    c = _case(m, k, n, "float32", True, "float32", seed=4)
+    c["xzp"] = torch.tensor([zp], dtype=torch.int32)
+    g = torch.Generator().manual_seed(3)
+    bufs = tuple(torch.randn(m, n, generator=g) for p in post if p in (O.POST_MUL, O.POST_ADD))
+    _compare(_run(capi, c, post, bufs), _oracle(c, post, bufs), f"zp={zp} post={post}")
+
+
 # ---- torch.ops.zentorch.zentorch_qlinear* -----------------------------------------------------------------
 def test_torch_ops_match_oracle(capi):
     ops = torch.ops.zentorch

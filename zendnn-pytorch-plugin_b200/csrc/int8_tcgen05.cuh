@@ -18,6 +18,10 @@
 //               quarter, each taking every other 32-column chunk), scale, bias, post-op, cast,
 //               16-byte stores
 //
+// The roles' control flow is uniform across their warp (see tc05.cuh) and the issuer looks at the next stage's
+// barrier while it issues: M = 1 on 8192 -> 10240 25.5 -> 22.4 us; M = 512 and larger, bound by operand delivery out of L2
+// and by power, did not change.
+//
 // Ring stages are recycled through full/empty mbarriers (tcgen05.commit frees a stage when the MMAs
 // that read it retire); accumulator buffers through tmem_full/tmem_empty mbarriers.  Every wait is
 // bounded: on expiry the role records a status code and stops, the other roles run into their own
@@ -72,6 +76,19 @@ struct SmemLayout {
   static constexpr int kTotal = kTileBytes + kVecBytes + kBarBytes + 1024;  // + slack to align to 1024
 };
 
+// A post-op chain on `n` (up to 32) consecutive outputs of one row.  The chain's code exists once, in a loop: unrolled over
+// the 32 values (and its four steps) it is some hundred kilobytes of instructions that a tile walks through once, which
+// made a 384 x 4096 x 1024 call of the static form take 55 us with 3 % of the issue slots used (13.8 us now).
+__device__ __forceinline__ void post_chain(float (&v)[32], const PostOpsDev &post, int64_t base, int n, int dtype) {
+  float w[32];          // indexed by the loop, so it lives in local memory; `v` stays in registers
+#pragma unroll
+  for (int j = 0; j < 32; ++j) w[j] = v[j];
+#pragma unroll 1
+  for (int j = 0; j < n; ++j) w[j] = apply_post_ops(w[j], post, base + j, dtype);
+#pragma unroll
+  for (int j = 0; j < 32; ++j) v[j] = w[j];
+}
+
 // Scale, bias and post-op for 32 consecutive outputs of one row, then the store.
 template <int UNARY>
 __device__ __forceinline__ void finish_chunk(const TcParams &p, const uint32_t (&r)[32], float s_m, int zp_m,
@@ -114,9 +131,7 @@ __device__ __forceinline__ void finish_chunk(const TcParams &p, const uint32_t (
 #pragma unroll
     for (int j = 0; j < 32; ++j) v[j] = unary_post(v[j], UNARY);
   } else {
-#pragma unroll
-    for (int j = 0; j < 32; ++j)
-      if (nb + j < p.N) v[j] = apply_post_ops(v[j], p.post, base + j, p.y_dtype);
+    post_chain(v, p.post, base, min(32, p.N - nb), p.y_dtype);
   }
   const bool full = nb + 32 <= p.N;
   if (p.y_dtype == ZT_BF16) {
@@ -160,15 +175,18 @@ __device__ __forceinline__ void finish_chunk_static(const TcParams &p, const uin
                                                     const float *wscale, const float *bias, const int32_t *rowsum,
                                                     const OutQuant &oq, int m, int nb) {
   float v[32];
+  // |acc| and |zp * rowsum| of 8-bit operands stay below 2^31 for K <= 65536 (as in the dynamic form) when the zero point
+  // is one that 8 bits can hold; other zero points and longer rows take 64 bits
+  const bool narrow = p.K <= 65536 && zp_x >= 0 && zp_x <= 255;
 #pragma unroll
   for (int j = 0; j < 32; ++j) {
-    const float af = p.src_zp ? (float)((int64_t)(int32_t)r[j] - (int64_t)zp_x * rowsum[j]) : (float)(int32_t)r[j];
+    const float af = !p.src_zp ? (float)(int32_t)r[j]
+                     : narrow  ? (float)((int32_t)r[j] - zp_x * rowsum[j])
+                               : (float)((int64_t)(int32_t)r[j] - (int64_t)zp_x * rowsum[j]);
     v[j] = __fadd_rn(__fmul_rn(af, s_x * wscale[j]), bias[j]);
   }
   const int64_t base = (int64_t)m * p.N + nb;
-#pragma unroll
-  for (int j = 0; j < 32; ++j)
-    if (nb + j < p.N) v[j] = apply_post_ops(v[j], p.post, base + j, p.post_dtype);
+  if (p.post.n_ops > 0) post_chain(v, p.post, base, min(32, p.N - nb), p.post_dtype);
   const int64_t out = (int64_t)m * p.ldy + nb;
   const bool full = nb + 32 <= p.N;
   if (p.y_dtype == ZT_U8 || p.y_dtype == ZT_S8) {
@@ -242,7 +260,8 @@ __global__ void __launch_bounds__(kThreads, 1) int8_tcgen05_kernel(const __grid_
 
   constexpr int kAccCols = NBUF * MH * BN;
   constexpr uint32_t kTmemCols = kAccCols <= 32 ? 32 : kAccCols <= 64 ? 64 : kAccCols <= 128 ? 128 : kAccCols <= 256 ? 256 : 512;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = tc::uniform_warp(), lane = threadIdx.x & 31;
+  const bool leader = lane == 0;     // the producer and the issuer run as whole warps, lane 0 issuing
   const int num_kb = (p.K + kBK - 1) / kBK;
   const int total_tiles = p.m_tiles * p.n_tiles;
 
@@ -270,9 +289,8 @@ __global__ void __launch_bounds__(kThreads, 1) int8_tcgen05_kernel(const __grid_
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    if (lane == 0) {
-      uint32_t it = 0;  // ring position, runs across tiles
-      bool ok = true;
+    {
+      const uint32_t full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar), smem0 = smem_u32(smem);
       // First pass over the ring: the weight tiles do not depend on the preceding kernel, so they are
       // requested before the dependency wait and the activation tiles of the same stages after it.
       int pre = 0;
@@ -281,76 +299,83 @@ __global__ void __launch_bounds__(kThreads, 1) int8_tcgen05_kernel(const __grid_
         const int n0 = ((int)blockIdx.x / p.m_tiles) * BN;
         pre = num_kb < STAGES ? num_kb : STAGES;
         for (int kb = 0; kb < pre; ++kb) {
-          tc::mbar_expect_tx(&full_bar[kb], L::kStageBytes);
-          tc::tma_load_2d(smem + kb * L::kStageBytes + L::kABytes, &tmap_b, &full_bar[kb], kb * kBK, n0);
+          tc::expect_tx_if(leader, full0 + kb * 8, L::kStageBytes);
+          tc::load_2d_if(leader, smem0 + kb * L::kStageBytes + L::kABytes, &tmap_b, full0 + kb * 8, kb * kBK, n0);
         }
         grid_dependency_wait();
         for (int kb = 0; kb < pre; ++kb)
-          tc::tma_load_2d(smem + kb * L::kStageBytes, &tmap_a, &full_bar[kb], kb * kBK, m0);
-        it = (uint32_t)pre;
+          tc::load_2d_if(leader, smem0 + kb * L::kStageBytes, &tmap_a, full0 + kb * 8, kb * kBK, m0);
       }
+      uint32_t s = (uint32_t)pre % STAGES, ph = pre == STAGES ? 0u : 1u;   // ring slot, parity of its "free" barrier
+      bool ok = true;
       for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
         const int m0 = (tile % p.m_tiles) * (MH * kBM);
         const int n0 = (tile / p.m_tiles) * BN;
-        for (int kb = (tile == (int)blockIdx.x ? pre : 0); kb < num_kb; ++kb, ++it) {
-          const uint32_t s = it % STAGES;
-          const uint32_t ph = (it / STAGES) & 1;
-          if (!tc::mbar_wait(&empty_bar[s], ph ^ 1)) {
+        for (int kb = (tile == (int)blockIdx.x ? pre : 0); kb < num_kb; ++kb) {
+          ok = tc::warp_wait(empty0 + s * 8, ph);
+          if (!ok) {
             tc::report_timeout(p.status, kStatusProducerTimeout);
-            ok = false;
             break;
           }
-          unsigned char *a_dst = smem + s * L::kStageBytes;
-          unsigned char *b_dst = a_dst + L::kABytes;
-          tc::mbar_expect_tx(&full_bar[s], L::kStageBytes);
-          tc::tma_load_2d(a_dst, &tmap_a, &full_bar[s], kb * kBK, m0);
-          tc::tma_load_2d(b_dst, &tmap_b, &full_bar[s], kb * kBK, n0);
+          const uint32_t a_dst = smem0 + s * L::kStageBytes, bar = full0 + s * 8;
+          tc::expect_tx_if(leader, bar, L::kStageBytes);
+          tc::load_2d_if(leader, a_dst, &tmap_a, bar, kb * kBK, m0);
+          tc::load_2d_if(leader, a_dst + L::kABytes, &tmap_b, bar, kb * kBK, n0);
+          if (++s == STAGES) {
+            s = 0;
+            ph ^= 1;
+          }
         }
       }
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    {
       constexpr uint32_t idesc = tc::instr_desc(2u, A_SIGNED ? 1u : 0u, 1u, kBM, BN);
-      uint32_t it = 0;
-      bool ok = true;
+      const uint64_t d0 = tc::smem_desc_k_sw128(0);
+      const uint32_t desc_hi = (uint32_t)(d0 >> 32);
+      const uint32_t field0 = (uint32_t)d0 | ((smem_u32(smem) & 0x3FFFF) >> 4);
+      const uint32_t full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar);
+      uint32_t s = 0, ph = 0;
+      bool ok = true, ready = false;
       int local = 0;
       for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++local) {
         const uint32_t buf = (uint32_t)local % NBUF;
         const uint32_t use = (uint32_t)local / NBUF;  // how many times this buffer was used before
-        if (ok && !tc::mbar_wait(&tmem_empty[buf], (use & 1) ^ 1)) {
-          tc::report_timeout(p.status, kStatusMmaTimeout);
-          ok = false;
-        }
+        ok = ok && tc::warp_wait(smem_u32(&tmem_empty[buf]), (use & 1) ^ 1);
+        if (!ok) tc::report_timeout(p.status, kStatusMmaTimeout);
         tc::fence_after_sync();
         const uint32_t d_tmem = tmem_base + buf * (MH * BN);
-        for (int kb = 0; kb < num_kb && ok; ++kb, ++it) {
-          const uint32_t s = it % STAGES;
-          const uint32_t ph = (it / STAGES) & 1;
-          if (!tc::mbar_wait(&full_bar[s], ph)) {
+        for (int kb = 0; kb < num_kb && ok; ++kb) {
+          if (!ready) ok = tc::warp_wait(full0 + s * 8, ph);
+          if (!ok) {
             tc::report_timeout(p.status, kStatusMmaTimeout);
-            ok = false;
             break;
           }
           tc::fence_after_sync();
-          const uint32_t a_addr = smem_u32(smem + s * L::kStageBytes);
-          const uint64_t a_desc = tc::smem_desc_k_sw128(a_addr);
-          const uint64_t b_desc = tc::smem_desc_k_sw128(a_addr + L::kABytes);
+          const uint32_t a_lo = field0 + s * (L::kStageBytes >> 4), b_lo = a_lo + (L::kABytes >> 4), bar = empty0 + s * 8;
+          if (++s == STAGES) {
+            s = 0;
+            ph ^= 1;
+          }
+          // a look at the next stage, answered while the MMAs are being issued
+          const uint32_t next = tc::mbar_test_addr(full0 + s * 8, ph);
 #pragma unroll
           for (int h = 0; h < MH; ++h) {
 #pragma unroll
             for (int k = 0; k < kBK / 32; ++k) {
               // 32 bytes of K per instruction: advance both start addresses by 32 >> 4 = 2; the second
               // 128-row half of the A stage starts 128 * 128 bytes further (>> 4 = 1024)
-              tc::mma_i8(d_tmem + h * BN, a_desc + h * (kBM * kBK / 16) + 2 * k, b_desc + 2 * k, idesc,
-                         (kb > 0 || k > 0) ? 1u : 0u);
+              tc::mma_i8_if(leader, d_tmem + h * BN, tc::smem_desc_from_words(a_lo + h * (kBM * kBK / 16) + 2 * k, desc_hi),
+                            tc::smem_desc_from_words(b_lo + 2 * k, desc_hi), idesc, (kb > 0 || k > 0) ? 1u : 0u);
             }
           }
-          tc::mma_commit(&empty_bar[s]);
+          tc::mma_commit_if(leader, bar);
+          ready = __all_sync(0xffffffffu, next);
         }
         // Arrive on the accumulator barrier in every case so that the epilogue never waits for a
         // commit that will not come; after a timeout the result is garbage but the kernel ends.
-        tc::mma_commit(&tmem_full[buf]);
+        tc::mma_commit_if(leader, smem_u32(&tmem_full[buf]));
       }
     }
   } else {
@@ -388,10 +413,8 @@ __global__ void __launch_bounds__(kThreads, 1) int8_tcgen05_kernel(const __grid_
       // All epilogue threads: the vectors of this tile are visible, and everybody has finished
       // reading the vectors of the tile two back (same buffer).
       asm volatile("bar.sync 1, %0;" ::"n"(kEpiWarps * 32) : "memory");
-      if (ok && !tc::mbar_wait(&tmem_full[buf], use & 1)) {
-        tc::report_timeout(p.status, kStatusEpilogueTimeout);
-        ok = false;
-      }
+      ok = ok && tc::warp_wait(smem_u32(&tmem_full[buf]), use & 1);
+      if (!ok && leader) tc::report_timeout(p.status, kStatusEpilogueTimeout);
       tc::fence_after_sync();
 #pragma unroll 1
       for (int h = 0; h < MH; ++h) {
@@ -447,7 +470,7 @@ __global__ void __launch_bounds__(kThreads, 1) int8_tcgen05_kernel(const __grid_
       // this warp has drained its part of the accumulator buffer
       tc::fence_before_sync();
       __syncwarp();
-      if (lane == 0) tc::mbar_arrive(&tmem_empty[buf]);
+      tc::arrive_if(leader, smem_u32(&tmem_empty[buf]));
     }
   }
 

@@ -137,6 +137,67 @@ __device__ __forceinline__ void fence_after_sync() { asm volatile("tcgen05.fence
 // Makes generic-proxy writes to shared memory visible to the async proxy (TMA / tcgen05 reads).
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
+// The same without suspending.
+__device__ __forceinline__ uint32_t mbar_test_addr(uint32_t addr, uint32_t parity) {
+  uint32_t done;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(done)
+      : "r"(addr), "r"(parity)
+      : "memory");
+  return done;
+}
+
+// ---- whole-warp roles -----------------------------------------------------------------------------
+// Index of the warp, from a shuffle: the compiler then knows that branches on it are uniform across the warp and keeps
+// what a role computes (descriptors, barrier addresses) in uniform registers.
+__device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+// Whole-warp barrier wait and single-lane operations without divergent branches: a branch that only one lane takes
+// costs the warp far more here than the instruction behind it.
+__device__ __forceinline__ bool warp_wait(uint32_t bar_addr, uint32_t parity) {
+#pragma unroll 1
+  for (uint32_t i = 0; i < kSpinLimit; ++i) {
+    if (__all_sync(0xffffffffu, mbar_try_addr(bar_addr, parity))) return true;
+    if (i > 64) __nanosleep(64);
+  }
+  return false;
+}
+__device__ __forceinline__ bool warp_wait_idle(uint32_t bar_addr, uint32_t parity) {   // the same for waits that last
+#pragma unroll 1
+  for (uint32_t i = 0; i < kSpinLimit; ++i) {
+    if (__all_sync(0xffffffffu, mbar_try_addr(bar_addr, parity))) return true;
+    __nanosleep(200);
+  }
+  return false;
+}
+__device__ __forceinline__ void arrive_if(bool lane_does, uint32_t bar_addr) {
+  asm volatile("{.reg .pred p; setp.ne.b32 p, %0, 0; @p mbarrier.arrive.shared::cta.b64 _, [%1];}" ::"r"((uint32_t)lane_does),
+               "r"(bar_addr)
+               : "memory");
+}
+__device__ __forceinline__ void expect_tx_if(bool lane_does, uint32_t bar_addr, uint32_t bytes) {
+  asm volatile("{.reg .pred p; setp.ne.b32 p, %0, 0; @p mbarrier.arrive.expect_tx.shared::cta.b64 _, [%1], %2;}" ::"r"(
+                   (uint32_t)lane_does),
+               "r"(bar_addr), "r"(bytes)
+               : "memory");
+}
+__device__ __forceinline__ void load_2d_if(bool lane_does, uint32_t dst, const CUtensorMap *m, uint32_t bar, int c0, int c1) {
+  asm volatile(
+      "{.reg .pred p; setp.ne.b32 p, %0, 0;\n\t"
+      "@p cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%1], [%2, {%4, %5}], [%3];}" ::"r"(
+          (uint32_t)lane_does),
+      "r"(dst), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(c0), "r"(c1)
+      : "memory");
+}
+__device__ __forceinline__ void load_3d_if(bool lane_does, uint32_t dst, const CUtensorMap *m, uint32_t bar, int c0, int c1,
+                                           int c2) {
+  asm volatile(
+      "{.reg .pred p; setp.ne.b32 p, %0, 0;\n\t"
+      "@p cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%1], [%2, {%4, %5, %6}], [%3];}"
+      ::"r"((uint32_t)lane_does), "r"(dst), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
+      : "memory");
+}
+
 // ---- descriptors --------------------------------------------------------------------------------
 // Shared-memory matrix descriptor for a K-major operand tile stored as rows of 128 bytes with the
 // 128-byte swizzle (what a TMA load with CU_TENSOR_MAP_SWIZZLE_128B writes): 8-row groups are 1024
@@ -160,12 +221,19 @@ __host__ __device__ constexpr uint32_t instr_desc(uint32_t c_format, uint32_t a_
 }
 
 // ---- MMA ------------------------------------------------------------------------------------------
-__device__ __forceinline__ void mma_i8(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                       uint32_t accumulate) {
+__device__ __forceinline__ void mma_i8_if(bool lane_does, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                          uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"((uint32_t)lane_does)
+      : "memory");
+}
+__device__ __forceinline__ void mma_commit_if(bool lane_does, uint32_t bar_addr) {
+  asm volatile(
+      "{.reg .pred p; setp.ne.b32 p, %0, 0; @p tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%1];}" ::"r"(
+          (uint32_t)lane_does),
+      "r"(bar_addr)
       : "memory");
 }
 // A operand (128 rows, two bf16 of K per 32-bit column) in tensor memory.

@@ -105,52 +105,6 @@ struct TcParams {
   int staged_gpc, groups;
 };
 
-// Whole-warp barrier wait and single-lane operations without divergent branches: a branch that only one lane takes
-// costs the warp far more here than the instruction behind it.
-__device__ __forceinline__ bool warp_wait(uint32_t bar_addr, uint32_t parity) {
-#pragma unroll 1
-  for (uint32_t i = 0; i < tc::kSpinLimit; ++i) {
-    if (__all_sync(0xffffffffu, tc::mbar_try_addr(bar_addr, parity))) return true;
-    if (i > 64) __nanosleep(64);
-  }
-  return false;
-}
-__device__ __forceinline__ bool drain_wait(uint32_t bar_addr, uint32_t parity) {   // the same for waits that last
-#pragma unroll 1
-  for (uint32_t i = 0; i < tc::kSpinLimit; ++i) {
-    if (__all_sync(0xffffffffu, tc::mbar_try_addr(bar_addr, parity))) return true;
-    __nanosleep(200);
-  }
-  return false;
-}
-__device__ __forceinline__ void arrive_if(bool lane_does, uint32_t bar_addr) {
-  asm volatile("{.reg .pred p; setp.ne.b32 p, %0, 0; @p mbarrier.arrive.shared::cta.b64 _, [%1];}" ::"r"((uint32_t)lane_does),
-               "r"(bar_addr)
-               : "memory");
-}
-__device__ __forceinline__ void expect_tx_if(bool lane_does, uint32_t bar_addr, uint32_t bytes) {
-  asm volatile("{.reg .pred p; setp.ne.b32 p, %0, 0; @p mbarrier.arrive.expect_tx.shared::cta.b64 _, [%1], %2;}" ::"r"(
-                   (uint32_t)lane_does),
-               "r"(bar_addr), "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ void load_2d_if(bool lane_does, uint32_t dst, const CUtensorMap *m, uint32_t bar, int c0, int c1) {
-  asm volatile(
-      "{.reg .pred p; setp.ne.b32 p, %0, 0;\n\t"
-      "@p cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%1], [%2, {%4, %5}], [%3];}" ::"r"(
-          (uint32_t)lane_does),
-      "r"(dst), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(c0), "r"(c1)
-      : "memory");
-}
-__device__ __forceinline__ void load_3d_if(bool lane_does, uint32_t dst, const CUtensorMap *m, uint32_t bar, int c0, int c1,
-                                           int c2) {
-  asm volatile(
-      "{.reg .pred p; setp.ne.b32 p, %0, 0;\n\t"
-      "@p cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%1], [%2, {%4, %5, %6}], [%3];}"
-      ::"r"((uint32_t)lane_does), "r"(dst), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
-      : "memory");
-}
-
 struct TileInfo {
   int m0, rows, n0, expert;
 };
@@ -433,7 +387,7 @@ __global__ void __launch_bounds__(threads_for(TEAMS), 1) woq_tcgen05_kernel(cons
   uint64_t *last_full = tmem_empty + 2;      // accumulator of the CTA's last segment
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(last_full + 1);
 
-  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  const int warp = tc::uniform_warp(), lane = threadIdx.x & 31;
   // Programmatic dependent launch: packed weights and scales are read before the wait for the preceding
   // kernel, activations, partial sums and output after it.  The grouped form reads its tile list (made by the
   // routing kernels before it) at once, so it waits first.
@@ -492,18 +446,18 @@ __global__ void __launch_bounds__(threads_for(TEAMS), 1) woq_tcgen05_kernel(cons
         const TileInfo t = decode_tile(p, wk.tile, n_mt);
         const int row = t.expert * p.N + t.n0;     // rows of the stacked weight: expert * N + n0
         for (uint32_t c = wk.c0; c < wk.c1; ++c) {
-          ok = warp_wait(empty_p0 + s * 8, ph);
+          ok = tc::warp_wait(empty_p0 + s * 8, ph);
           if (!ok) {
             tc::report_timeout(p.status, kStatusProducerTimeout);
             break;
           }
           const uint32_t bar = full_p0 + s * 8;
           const int g0 = t.expert * p.groups + (int)((c * kChunkK) >> (p.gs_log2 & 31));
-          expect_tx_if(leader, bar, chunk_tx);
-          load_2d_if(leader, packed0 + s * kChunkBytes, &tmap_w, bar, (int)c * (kChunkK / 8), row);
+          tc::expect_tx_if(leader, bar, chunk_tx);
+          tc::load_2d_if(leader, packed0 + s * kChunkBytes, &tmap_w, bar, (int)c * (kChunkK / 8), row);
           if (p.staged_gpc) {
-            load_2d_if(leader, sc0 + s * kScaleSlotBytes, &tmap_s, bar, t.n0, g0);
-            if (kAsym) load_2d_if(leader, sc0 + s * kScaleSlotBytes + kZeroSlotOffset, &tmap_z, bar, t.n0, g0);
+            tc::load_2d_if(leader, sc0 + s * kScaleSlotBytes, &tmap_s, bar, t.n0, g0);
+            if (kAsym) tc::load_2d_if(leader, sc0 + s * kScaleSlotBytes + kZeroSlotOffset, &tmap_z, bar, t.n0, g0);
           }
           if (++s == PSTAGES) {
             s = 0;
@@ -526,18 +480,18 @@ __global__ void __launch_bounds__(threads_for(TEAMS), 1) woq_tcgen05_kernel(cons
         const uint32_t bytes = (uint32_t)(first ? p.x_box : p.x_box2) * (XK / 64) * 128u;
         int k = (int)wk.c0 * kChunkK;
         for (uint32_t i = 0; i < (wk.c1 - wk.c0) * (kChunkK / XK); ++i, k += XK) {
-          ok = warp_wait(empty0 + s * 8, ph);
+          ok = tc::warp_wait(empty0 + s * 8, ph);
           if (!ok) {
             tc::report_timeout(p.status, kStatusProducerTimeout);
             break;
           }
           const uint32_t bar = full0 + s * 8, dst = x0 + s * L::kXBytes;
           if (k >= p.K) {                     // void
-            arrive_if(leader, bar);
+            tc::arrive_if(leader, bar);
           } else {
-            expect_tx_if(leader, bar, bytes);
+            tc::expect_tx_if(leader, bar, bytes);
             // 64 k x rows x (XK / 64) in one copy: k past the end of K reads as zeros and is not multiplied
-            load_3d_if(leader, dst, map, bar, 0, t.m0, k >> 6);
+            tc::load_3d_if(leader, dst, map, bar, 0, t.m0, k >> 6);
           }
           if (++s == XSTAGES) {
             s = 0;
@@ -562,7 +516,7 @@ __global__ void __launch_bounds__(threads_for(TEAMS), 1) woq_tcgen05_kernel(cons
         const uint32_t buf = local & 1, use = local >> 1;
         ++local;
         const uint32_t idesc = tc::instr_desc(1u, 1u, 1u, kBN, (uint32_t)((t.rows + 15) & ~15));
-        ok = ok && warp_wait(smem_u32(&tmem_empty[buf]), (use & 1) ^ 1);
+        ok = ok && tc::warp_wait(smem_u32(&tmem_empty[buf]), (use & 1) ^ 1);
         if (!ok) tc::report_timeout(p.status, kStatusMmaTimeout);
         tc::fence_after_sync();
         const uint32_t d_tmem = tmem_base + buf * NMAX;
@@ -572,7 +526,7 @@ __global__ void __launch_bounds__(threads_for(TEAMS), 1) woq_tcgen05_kernel(cons
         const uint32_t block = (uint32_t)(t.rows <= p.x_box ? p.x_box : p.x_box2) * 8u;   // 64 k of the tile, in 16 bytes
         for (uint32_t i = 0; i < stages && ok; ++i, k += KS) {
           if (!ready) {
-            ok = warp_wait(full_x0 + xs * 8, xph) && warp_wait(full_a0 + s * 8, ph);
+            ok = tc::warp_wait(full_x0 + xs * 8, xph) && tc::warp_wait(full_a0 + s * 8, ph);
             if (!ok) {
               tc::report_timeout(p.status, kStatusMmaTimeout);
               break;
@@ -644,7 +598,7 @@ __global__ void __launch_bounds__(threads_for(TEAMS), 1) woq_tcgen05_kernel(cons
     // one stage: `param()` gives the dequantisation parameters of its 32-k pieces, one after the other
     auto convert_stage = [&](int quads, auto &&param) {
       // also for a void stage: its arrival below must not run ahead of the slot's previous round
-      ok = ok && warp_wait(empty_a0 + slot * 8, e_ph);
+      ok = ok && tc::warp_wait(empty_a0 + slot * 8, e_ph);
       tc::fence_after_sync();
       if (ok && quads > 0) {
         // One copy of the conversion code, a 16-byte piece of the row per iteration: the teams are at different
@@ -663,8 +617,8 @@ __global__ void __launch_bounds__(threads_for(TEAMS), 1) woq_tcgen05_kernel(cons
       tc::tmem_st_wait();
       tc::fence_before_sync();
       __syncwarp();
-      arrive_if(lane == 0, full_a0 + slot * 8);
-      arrive_if(lane == 0, smem_u32(&empty_p[ps]));
+      tc::arrive_if(lane == 0, full_a0 + slot * 8);
+      tc::arrive_if(lane == 0, smem_u32(&empty_p[ps]));
       slot += TEAMS;
       if (slot >= SLOTS) {
         slot = team;
@@ -684,7 +638,7 @@ __global__ void __launch_bounds__(threads_for(TEAMS), 1) woq_tcgen05_kernel(cons
       // groups are at least 128 k wide: one scale per stage, in the chunk's slot
       const uint32_t sc_off = ((p.staged_gpc == 2 ? (j * KS) >> 7 : 0u) * kBN + row) * (kScaleDtype == ZT_F32 ? 4 : 2);
       for (; left > 0; --left) {
-        ok = ok && warp_wait(smem_u32(&full_p[ps]), pph);
+        ok = ok && tc::warp_wait(smem_u32(&full_p[ps]), pph);
         const unsigned char *slot = sc_ring + ps * kScaleSlotBytes + sc_off;
         const DqParam d = dq_param<MODE>(load_as_float(slot, 0, kScaleDtype),
                                          kAsym ? load_as_float(slot + kZeroSlotOffset, 0, kScaleDtype) : 0.f);
@@ -742,7 +696,7 @@ __global__ void __launch_bounds__(threads_for(TEAMS), 1) woq_tcgen05_kernel(cons
 #pragma unroll
         for (int u = 0; u < kSub; ++u) d[u] = dq_param<MODE>(ns[u], kAsym ? nz[u] : 0.f);
         fetch();
-        ok = ok && warp_wait(smem_u32(&full_p[ps]), pph);
+        ok = ok && tc::warp_wait(smem_u32(&full_p[ps]), pph);
         convert_stage(ok ? min(kSub, (p.K - (int)(c * kChunkK + j * KS)) / 32) : 0, [&]() {
           const DqParam first = d[0];
 #pragma unroll
@@ -795,7 +749,7 @@ __global__ void __launch_bounds__(threads_for(TEAMS), 1) woq_tcgen05_kernel(cons
       cta_last = wd.cta_of(wd.tile * wd.chunks + wd.chunks - 1);
       first_slot = wd.first_of(cta_first) < wd.tile * wd.chunks ? 1u : 0u;
     }
-    ok = ok && drain_wait(last ? smem_u32(last_full) : smem_u32(&tmem_full[buf]), last ? 0u : (use & 1));
+    ok = ok && tc::warp_wait_idle(last ? smem_u32(last_full) : smem_u32(&tmem_full[buf]), last ? 0u : (use & 1));
     if (!ok && lane == 0) tc::report_timeout(p.status, kStatusEpilogueTimeout);
     tc::fence_after_sync();
     const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + buf * NMAX;
@@ -932,7 +886,7 @@ __global__ void __launch_bounds__(threads_for(TEAMS), 1) woq_tcgen05_kernel(cons
     if (!last) {
       tc::fence_before_sync();
       __syncwarp();
-      arrive_if(lane == 0, smem_u32(&tmem_empty[buf]));
+      tc::arrive_if(lane == 0, smem_u32(&tmem_empty[buf]));
     }
   }
   }
