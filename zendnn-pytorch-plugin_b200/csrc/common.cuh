@@ -155,10 +155,12 @@ struct PostOpsDev {
 inline PostOpsDev to_dev(const zt_post_ops_t &p) {
   PostOpsDev d{};
   d.n_ops = p.n_ops;
+  int operands = 0;   // buffers past those that the chain reads stay null, whatever the caller left there
   for (int i = 0; i < ZT_MAX_POST_OPS; ++i) {
     d.ids[i] = p.ids[i];
-    d.bufs[i] = p.buffers[i];
+    if (i < p.n_ops && (p.ids[i] == ZT_POST_MUL || p.ids[i] == ZT_POST_ADD)) ++operands;
   }
+  for (int i = 0; i < operands; ++i) d.bufs[i] = p.buffers[i];
   return d;
 }
 
