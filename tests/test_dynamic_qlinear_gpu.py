@@ -183,3 +183,27 @@ def test_cta_pair_tiles_match_the_one_cta_kernel(capi, bn):
     assert torch.equal(got, expect)
     ref = O.dynamic_qlinear(x.cpu(), w.cpu(), ws.cpu(), b.cpu(), post_ops=[O.POST_ADD], buffers=[add.cpu()])
     assert_close_bf16(got, ref, what=f"pair tile {bn} vs oracle")
+
+
+@pytest.mark.parametrize("bn", [16, 48, 80, 144, 240, 1016, 1080, 1208, 1240])
+@pytest.mark.parametrize("m,k,n", [(1, 640, 300), (16, 1024, 515), (17, 144, 97), (113, 384, 250), (200, 1408, 481)])
+def test_tile_widths_and_k_groups(capi, bn, m, k, n):
+    """Every width is a run-time argument: odd multiples of 16 end a tile inside a 32-column chunk; few rows are loaded
+    alone; up to four 128-byte blocks of K share a stage (K = 640: the second stage is three quarters past the end,
+    K = 144: no multiple of 128).  Sums bit for bit, and the bf16 / fp32 epilogue against a 64-bit evaluation."""
+    if bn >= 1000 and m <= 128:
+        pytest.skip("256-row tiles are for more than 128 rows")
+    g = torch.Generator().manual_seed(m + k + n)
+    q = torch.randint(-128, 128, (m, k), generator=g, dtype=torch.int8)
+    w = torch.randint(-128, 128, (n, k), generator=g, dtype=torch.int8)
+    algo = capi.ZT_ALGO_TCGEN05 | (bn << 8)
+    acc = capi.int8_gemm_s32(q.cuda(), w.cuda(), algo=algo).cpu()
+    assert torch.equal(acc.double(), q.double() @ w.double().t())
+    for dt in (torch.bfloat16, torch.float32):
+        x, w8, ws, b = [t.cuda() for t in make_int8_case(m, k, n, seed=m, x_dtype=dt)]
+        y = capi.dynamic_qlinear(x, w8, ws, b, algo=algo).cpu()
+        qx, sx, _ = (t.cpu() for t in capi.dynamic_quantize(x))
+        exact = (qx.double() @ w8.cpu().double().t()) * sx.double().unsqueeze(1) * ws.cpu().double() + b.cpu().double()
+        # bf16 rounds to 2^-9 of the value; fp32: three roundings of 2^-24, relative to the terms of the final sum
+        bound = 2 ** -8 * exact.abs() + 1e-6 if dt == torch.bfloat16 else 2 ** -21 * (exact.abs() + b.cpu().double().abs() + 1e-3)
+        assert ((y.double() - exact).abs() <= bound).all(), (bn, m, k, n, dt)

@@ -4,13 +4,13 @@
 //   Y = post_ops( (acc - zp_m * wsum_n) * (s_m * w_n) + bias_n )
 //
 // Both operands are K-major, so they go from global memory to shared memory with plain 2-D TMA tile
-// loads (128 bytes of K per row, 128-byte swizzle) and are consumed in place by
-// tcgen05.mma.kind::i8 (K = 32 per instruction, four per 128-byte k-block).  The kernel is
+// loads (128 bytes of K per row, 128-byte swizzle; up to four such blocks of K per stage for small tiles) and are
+// consumed in place by tcgen05.mma.kind::i8 (K = 32 per instruction, four per 128-byte block).  The kernel is
 // persistent: one CTA per SM walks over (MH*128) x BN output tiles (MH = 2 reuses each weight
 // stage for two 128-row accumulators, which halves the weight bytes pulled per MAC) (tiles that share a weight column
 // block are adjacent in the order, so they run at the same time on neighbouring SMs and the weight
-// block is fetched from HBM once).  The int32 accumulator lives in tensor memory and is double
-// buffered, so the epilogue of tile i overlaps the main loop of tile i+1:
+// block is fetched from HBM once).  The tile's width BN is a run-time argument (pick_tile in int8_tcgen05.cu).  The
+// int32 accumulator lives in tensor memory and is double buffered up to 512 columns in all, so the epilogue of tile i overlaps the main loop of tile i+1:
 //
 //   warp 0      TMA producer (one lane): fills the shared-memory ring, across tile boundaries
 //   warp 1      allocates tensor memory, issues the MMAs (one lane), frees tensor memory
@@ -44,9 +44,15 @@ constexpr int kThreads = 64 + kEpiWarps * 32;
 // requantised or strided output); kept apart so that the dynamic form's epilogue carries none of it
 enum EpiMode { kEpiS32 = 0, kEpiLinear = 1, kEpiStatic = 2 };
 
+constexpr int kMaxBN = 256;
+constexpr int kMaxStages = 24;
+
 struct TcParams {
   int M, N, K;
   int m_tiles, n_tiles;
+  // tile and ring, chosen by the host (see pick_tile): tile width (a multiple of 16), accumulator buffers, rows of an
+  // activation box (MH * 128, or fewer when the call has fewer), ring stages, 128-byte blocks of K per stage, stage size
+  int bn, nbuf, a_rows, stages, group, stage_bytes;
   // epilogue
   const float *src_scale;  // [M]
   const int32_t *src_zp;   // [M] or null
@@ -65,16 +71,19 @@ struct TcParams {
   int64_t ldy;
 };
 
-template <int MH, int BN, int STAGES>
-struct SmemLayout {
-  static constexpr int kABytes = MH * kBM * kBK;
-  static constexpr int kBBytes = BN * kBK;
-  static constexpr int kStageBytes = kABytes + kBBytes;
-  static constexpr int kTileBytes = STAGES * kStageBytes;
-  static constexpr int kVecBytes = 2 * 3 * BN * 4;      // per accumulator buffer: w_scale, bias, rowsum
-  static constexpr int kBarBytes = (2 * STAGES + 4) * 8 + 8;
-  static constexpr int kTotal = kTileBytes + kVecBytes + kBarBytes + 1024;  // + slack to align to 1024
-};
+// Dynamic shared memory: the ring, then the vectors and the barriers.  The MMA always reads MH * 128 rows of A; with
+// fewer in a stage it runs on into what follows (rows that are never stored), so the ring is padded to keep that inside.
+constexpr int kVecBytes = 2 * 3 * kMaxBN * 4;            // per accumulator buffer: w_scale, bias, rowsum
+constexpr int kBarBytes = (2 * kMaxStages + 4) * 8 + 8;
+constexpr int kSmemLimit = 227 * 1024;
+// Columns of tensor memory of a 128-row accumulator.
+__host__ __device__ constexpr int acc_stride(int bn) { return (bn + 31) & ~31; }
+__host__ __device__ constexpr int ring_pad(int mh, int stage_bytes) {
+  return mh * kBM * kBK > stage_bytes ? mh * kBM * kBK - stage_bytes : 0;
+}
+__host__ __device__ constexpr int smem_bytes(int mh, int stages, int stage_bytes) {
+  return stages * stage_bytes + ring_pad(mh, stage_bytes) + kVecBytes + kBarBytes + 1024;   // + slack to align to 1024
+}
 
 // A post-op chain on `n` (up to 32) consecutive outputs of one row.  The chain's code exists once, in a loop: unrolled over
 // the 32 values (and its four steps) it is some hundred kilobytes of instructions that a tile walks through once, which
@@ -89,11 +98,46 @@ __device__ __forceinline__ void post_chain(float (&v)[32], const PostOpsDev &pos
   for (int j = 0; j < 32; ++j) v[j] = w[j];
 }
 
+__device__ __forceinline__ uint4 pack_bf16x8(const float *v) {
+  __nv_bfloat162 t0 = __floats2bfloat162_rn(v[0], v[1]);
+  __nv_bfloat162 t1 = __floats2bfloat162_rn(v[2], v[3]);
+  __nv_bfloat162 t2 = __floats2bfloat162_rn(v[4], v[5]);
+  __nv_bfloat162 t3 = __floats2bfloat162_rn(v[6], v[7]);
+  return make_uint4(*reinterpret_cast<uint32_t *>(&t0), *reinterpret_cast<uint32_t *>(&t1),
+                    *reinterpret_cast<uint32_t *>(&t2), *reinterpret_cast<uint32_t *>(&t3));
+}
+// `left` (at most 32) consecutive outputs of one row, in 16-byte stores where `vec` says that the row allows them.
+__device__ __forceinline__ void store_bf16(__nv_bfloat16 *dst, const float (&v)[32], int left, bool vec) {
+  if (vec && left >= 32) {
+#pragma unroll
+    for (int j = 0; j < 32; j += 8) *reinterpret_cast<uint4 *>(dst + j) = pack_bf16x8(v + j);
+  } else if (vec && left >= 16 && (left & 7) == 0) {      // a tile whose width is an odd multiple of 16
+#pragma unroll
+    for (int j = 0; j < 32; j += 8)
+      if (j < left) *reinterpret_cast<uint4 *>(dst + j) = pack_bf16x8(v + j);
+  } else {
+#pragma unroll
+    for (int j = 0; j < 32; ++j)
+      if (j < left) dst[j] = __float2bfloat16_rn(v[j]);
+  }
+}
+__device__ __forceinline__ void store_f32(float *dst, const float (&v)[32], int left, bool vec) {
+  if (vec && (left >= 32 || (left & 3) == 0)) {
+#pragma unroll
+    for (int j = 0; j < 32; j += 4)
+      if (j < left) *reinterpret_cast<float4 *>(dst + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+  } else {
+#pragma unroll
+    for (int j = 0; j < 32; ++j)
+      if (j < left) dst[j] = v[j];
+  }
+}
+
 // Scale, bias and post-op for 32 consecutive outputs of one row, then the store.
 template <int UNARY>
 __device__ __forceinline__ void finish_chunk(const TcParams &p, const uint32_t (&r)[32], float s_m, int zp_m,
                                              const float *wscale, const float *bias, const int32_t *rowsum, int m,
-                                             int nb) {
+                                             int nb, int n_end) {
   float v[32];
   // per-column vectors of the chunk, read as 16-byte shared loads (same address in every lane: broadcast)
   float wsc[32], bia[32];
@@ -131,40 +175,13 @@ __device__ __forceinline__ void finish_chunk(const TcParams &p, const uint32_t (
 #pragma unroll
     for (int j = 0; j < 32; ++j) v[j] = unary_post(v[j], UNARY);
   } else {
-    post_chain(v, p.post, base, min(32, p.N - nb), p.y_dtype);
+    post_chain(v, p.post, base, min(32, n_end - nb), p.y_dtype);
   }
-  const bool full = nb + 32 <= p.N;
+  const int left = n_end - nb;             // columns of the chunk that belong to the tile
   if (p.y_dtype == ZT_BF16) {
-    __nv_bfloat16 *dst = reinterpret_cast<__nv_bfloat16 *>(p.y) + base;
-    if (full && (p.N & 7) == 0) {
-#pragma unroll
-      for (int j = 0; j < 32; j += 8) {
-        uint4 o;
-        __nv_bfloat162 t0 = __floats2bfloat162_rn(v[j], v[j + 1]);
-        __nv_bfloat162 t1 = __floats2bfloat162_rn(v[j + 2], v[j + 3]);
-        __nv_bfloat162 t2 = __floats2bfloat162_rn(v[j + 4], v[j + 5]);
-        __nv_bfloat162 t3 = __floats2bfloat162_rn(v[j + 6], v[j + 7]);
-        o.x = *reinterpret_cast<uint32_t *>(&t0);
-        o.y = *reinterpret_cast<uint32_t *>(&t1);
-        o.z = *reinterpret_cast<uint32_t *>(&t2);
-        o.w = *reinterpret_cast<uint32_t *>(&t3);
-        *reinterpret_cast<uint4 *>(dst + j) = o;
-      }
-    } else {
-#pragma unroll
-      for (int j = 0; j < 32; ++j)
-        if (nb + j < p.N) dst[j] = __float2bfloat16_rn(v[j]);
-    }
+    store_bf16(reinterpret_cast<__nv_bfloat16 *>(p.y) + base, v, left, (p.N & 7) == 0);
   } else {
-    float *dst = reinterpret_cast<float *>(p.y) + base;
-    if (full && (p.N & 3) == 0) {
-#pragma unroll
-      for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4 *>(dst + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-    } else {
-#pragma unroll
-      for (int j = 0; j < 32; ++j)
-        if (nb + j < p.N) dst[j] = v[j];
-    }
+    store_f32(reinterpret_cast<float *>(p.y) + base, v, left, (p.N & 3) == 0);
   }
 }
 
@@ -173,7 +190,7 @@ __device__ __forceinline__ void finish_chunk(const TcParams &p, const uint32_t (
 // requantises or honours a row stride.
 __device__ __forceinline__ void finish_chunk_static(const TcParams &p, const uint32_t (&r)[32], float s_x, int zp_x,
                                                     const float *wscale, const float *bias, const int32_t *rowsum,
-                                                    const OutQuant &oq, int m, int nb) {
+                                                    const OutQuant &oq, int m, int nb, int n_end) {
   float v[32];
   // |acc| and |zp * rowsum| of 8-bit operands stay below 2^31 for K <= 65536 (as in the dynamic form) when the zero point
   // is one that 8 bits can hold; other zero points and longer rows take 64 bits
@@ -186,14 +203,15 @@ __device__ __forceinline__ void finish_chunk_static(const TcParams &p, const uin
     v[j] = __fadd_rn(__fmul_rn(af, s_x * wscale[j]), bias[j]);
   }
   const int64_t base = (int64_t)m * p.N + nb;
-  if (p.post.n_ops > 0) post_chain(v, p.post, base, min(32, p.N - nb), p.post_dtype);
+  if (p.post.n_ops > 0) post_chain(v, p.post, base, min(32, n_end - nb), p.post_dtype);
   const int64_t out = (int64_t)m * p.ldy + nb;
-  const bool full = nb + 32 <= p.N;
+  const int left = n_end - nb;
   if (p.y_dtype == ZT_U8 || p.y_dtype == ZT_S8) {
     uint8_t *dst = reinterpret_cast<uint8_t *>(p.y) + out;
-    if (full && ((reinterpret_cast<uintptr_t>(dst)) & 15) == 0) {
+    const bool vec = (reinterpret_cast<uintptr_t>(dst) & 15) == 0;
 #pragma unroll
-      for (int j = 0; j < 32; j += 16) {
+    for (int j = 0; j < 32; j += 16) {
+      if (vec && j + 16 <= left) {
         uint32_t w4[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -202,67 +220,52 @@ __device__ __forceinline__ void finish_chunk_static(const TcParams &p, const uin
           for (int b = 0; b < 4; ++b) w4[q] |= ((uint32_t)requantize(v[j + 4 * q + b], oq) & 0xffu) << (8 * b);
         }
         *reinterpret_cast<uint4 *>(dst + j) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
-      }
-    } else {
+      } else {
 #pragma unroll
-      for (int j = 0; j < 32; ++j)
-        if (nb + j < p.N) dst[j] = (uint8_t)requantize(v[j], oq);
+        for (int e = 0; e < 16; ++e)
+          if (j + e < left) dst[j + e] = (uint8_t)requantize(v[j + e], oq);
+      }
     }
   } else if (p.y_dtype == ZT_BF16) {
     __nv_bfloat16 *dst = reinterpret_cast<__nv_bfloat16 *>(p.y) + out;
-    if (full && ((reinterpret_cast<uintptr_t>(dst)) & 15) == 0) {
-#pragma unroll
-      for (int j = 0; j < 32; j += 8) {
-        uint4 o;
-        __nv_bfloat162 t0 = __floats2bfloat162_rn(v[j], v[j + 1]);
-        __nv_bfloat162 t1 = __floats2bfloat162_rn(v[j + 2], v[j + 3]);
-        __nv_bfloat162 t2 = __floats2bfloat162_rn(v[j + 4], v[j + 5]);
-        __nv_bfloat162 t3 = __floats2bfloat162_rn(v[j + 6], v[j + 7]);
-        o.x = *reinterpret_cast<uint32_t *>(&t0);
-        o.y = *reinterpret_cast<uint32_t *>(&t1);
-        o.z = *reinterpret_cast<uint32_t *>(&t2);
-        o.w = *reinterpret_cast<uint32_t *>(&t3);
-        *reinterpret_cast<uint4 *>(dst + j) = o;
-      }
-    } else {
-#pragma unroll
-      for (int j = 0; j < 32; ++j)
-        if (nb + j < p.N) dst[j] = __float2bfloat16_rn(v[j]);
-    }
+    store_bf16(dst, v, left, (reinterpret_cast<uintptr_t>(dst) & 15) == 0);
   } else {
     float *dst = reinterpret_cast<float *>(p.y) + out;
-    if (full && ((reinterpret_cast<uintptr_t>(dst)) & 15) == 0) {
-#pragma unroll
-      for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4 *>(dst + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-    } else {
-#pragma unroll
-      for (int j = 0; j < 32; ++j)
-        if (nb + j < p.N) dst[j] = v[j];
-    }
+    store_f32(dst, v, left, (reinterpret_cast<uintptr_t>(dst) & 15) == 0);
   }
 }
 
-template <int MH, int BN, int STAGES, int NBUF, int EPI, bool A_SIGNED>
+// One operand of a stage: `group` blocks of 128 bytes of K, one copy (a two-dimensional map for one block, which also takes a
+// K that is no multiple of 128).
+__device__ __forceinline__ void load_stage(bool leader, int group, uint32_t dst, const CUtensorMap *m, uint32_t bar, int kb, int row) {
+  if (group == 1)
+    tc::load_2d_if(leader, dst, m, bar, kb * kBK, row);
+  else
+    tc::load_3d_if(leader, dst, m, bar, 0, row, kb * group);
+}
+
+template <int MH, int EPI, bool A_SIGNED>
 __global__ void __launch_bounds__(kThreads, 1) int8_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
                                                                    const __grid_constant__ CUtensorMap tmap_b,
                                                                    const TcParams p) {
-  using L = SmemLayout<MH, BN, STAGES>;
-  static_assert(NBUF * MH * BN <= 512, "accumulators exceed tensor memory");
   extern __shared__ unsigned char smem_dyn[];
   // align on the shared-window address (what the descriptors and TMA see), not the generic one
   unsigned char *smem = smem_dyn + ((1024u - (smem_u32(smem_dyn) & 1023u)) & 1023u);
-  float *s_vec = reinterpret_cast<float *>(smem + L::kTileBytes);  // [2][3][BN]
-  uint64_t *full_bar = reinterpret_cast<uint64_t *>(smem + L::kTileBytes + L::kVecBytes);
-  uint64_t *empty_bar = full_bar + STAGES;
-  uint64_t *tmem_full = empty_bar + STAGES;   // [2]
+  const int BN = p.bn, STAGES = p.stages;
+  const uint32_t stage_bytes = (uint32_t)p.stage_bytes, a_bytes = (uint32_t)(p.a_rows * p.group) * kBK, NBUF = (uint32_t)p.nbuf;
+  unsigned char *after_ring = smem + STAGES * stage_bytes + ring_pad(MH, p.stage_bytes);
+  float *s_vec = reinterpret_cast<float *>(after_ring);  // [2][3][kMaxBN]
+  uint64_t *full_bar = reinterpret_cast<uint64_t *>(after_ring + kVecBytes);
+  uint64_t *empty_bar = full_bar + kMaxStages;
+  uint64_t *tmem_full = empty_bar + kMaxStages;   // [2]
   uint64_t *tmem_empty = tmem_full + 2;       // [2]
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(tmem_empty + 2);
 
-  constexpr int kAccCols = NBUF * MH * BN;
-  constexpr uint32_t kTmemCols = kAccCols <= 32 ? 32 : kAccCols <= 64 ? 64 : kAccCols <= 128 ? 128 : kAccCols <= 256 ? 256 : 512;
+  constexpr uint32_t kTmemCols = 512;
+  const uint32_t acc_cols = (uint32_t)acc_stride(BN);
   const int warp = tc::uniform_warp(), lane = threadIdx.x & 31;
   const bool leader = lane == 0;     // the producer and the issuer run as whole warps, lane 0 issuing
-  const int num_kb = (p.K + kBK - 1) / kBK;
+  const int num_kb = (p.K + kBK * p.group - 1) / (kBK * p.group);   // stages per tile (K past the end reads as zeros)
   const int total_tiles = p.m_tiles * p.n_tiles;
 
   if (threadIdx.x == 0) {
@@ -299,14 +302,14 @@ __global__ void __launch_bounds__(kThreads, 1) int8_tcgen05_kernel(const __grid_
         const int n0 = ((int)blockIdx.x / p.m_tiles) * BN;
         pre = num_kb < STAGES ? num_kb : STAGES;
         for (int kb = 0; kb < pre; ++kb) {
-          tc::expect_tx_if(leader, full0 + kb * 8, L::kStageBytes);
-          tc::load_2d_if(leader, smem0 + kb * L::kStageBytes + L::kABytes, &tmap_b, full0 + kb * 8, kb * kBK, n0);
+          tc::expect_tx_if(leader, full0 + kb * 8, stage_bytes);
+          load_stage(leader, p.group, smem0 + kb * stage_bytes + a_bytes, &tmap_b, full0 + kb * 8, kb, n0);
         }
         grid_dependency_wait();
         for (int kb = 0; kb < pre; ++kb)
-          tc::load_2d_if(leader, smem0 + kb * L::kStageBytes, &tmap_a, full0 + kb * 8, kb * kBK, m0);
+          load_stage(leader, p.group, smem0 + kb * stage_bytes, &tmap_a, full0 + kb * 8, kb, m0);
       }
-      uint32_t s = (uint32_t)pre % STAGES, ph = pre == STAGES ? 0u : 1u;   // ring slot, parity of its "free" barrier
+      uint32_t s = pre == STAGES ? 0u : (uint32_t)pre, ph = pre == STAGES ? 0u : 1u;   // ring slot, parity of its "free" barrier
       bool ok = true;
       for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
         const int m0 = (tile % p.m_tiles) * (MH * kBM);
@@ -317,11 +320,11 @@ __global__ void __launch_bounds__(kThreads, 1) int8_tcgen05_kernel(const __grid_
             tc::report_timeout(p.status, kStatusProducerTimeout);
             break;
           }
-          const uint32_t a_dst = smem0 + s * L::kStageBytes, bar = full0 + s * 8;
-          tc::expect_tx_if(leader, bar, L::kStageBytes);
-          tc::load_2d_if(leader, a_dst, &tmap_a, bar, kb * kBK, m0);
-          tc::load_2d_if(leader, a_dst + L::kABytes, &tmap_b, bar, kb * kBK, n0);
-          if (++s == STAGES) {
+          const uint32_t a_dst = smem0 + s * stage_bytes, bar = full0 + s * 8;
+          tc::expect_tx_if(leader, bar, stage_bytes);
+          load_stage(leader, p.group, a_dst, &tmap_a, bar, kb, m0);
+          load_stage(leader, p.group, a_dst + a_bytes, &tmap_b, bar, kb, n0);
+          if (++s == (uint32_t)STAGES) {
             s = 0;
             ph ^= 1;
           }
@@ -331,21 +334,22 @@ __global__ void __launch_bounds__(kThreads, 1) int8_tcgen05_kernel(const __grid_
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
     {
-      constexpr uint32_t idesc = tc::instr_desc(2u, A_SIGNED ? 1u : 0u, 1u, kBM, BN);
+      const uint32_t idesc = tc::instr_desc(2u, A_SIGNED ? 1u : 0u, 1u, kBM, (uint32_t)BN);
       const uint64_t d0 = tc::smem_desc_k_sw128(0);
       const uint32_t desc_hi = (uint32_t)(d0 >> 32);
       const uint32_t field0 = (uint32_t)d0 | ((smem_u32(smem) & 0x3FFFF) >> 4);
       const uint32_t full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar);
+      const uint32_t a_block = (uint32_t)p.a_rows * (kBK / 16), b_block = (uint32_t)BN * (kBK / 16);   // a 128-byte block of K
       uint32_t s = 0, ph = 0;
       bool ok = true, ready = false;
       int local = 0;
       for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++local) {
-        const uint32_t buf = (uint32_t)local % NBUF;
-        const uint32_t use = (uint32_t)local / NBUF;  // how many times this buffer was used before
+        const uint32_t buf = NBUF == 2 ? (uint32_t)local & 1u : 0u;
+        const uint32_t use = NBUF == 2 ? (uint32_t)local >> 1 : (uint32_t)local;  // how many times this buffer was used before
         ok = ok && tc::warp_wait(smem_u32(&tmem_empty[buf]), (use & 1) ^ 1);
         if (!ok) tc::report_timeout(p.status, kStatusMmaTimeout);
         tc::fence_after_sync();
-        const uint32_t d_tmem = tmem_base + buf * (MH * BN);
+        const uint32_t d_tmem = tmem_base + buf * (MH * acc_cols);
         for (int kb = 0; kb < num_kb && ok; ++kb) {
           if (!ready) ok = tc::warp_wait(full0 + s * 8, ph);
           if (!ok) {
@@ -353,21 +357,25 @@ __global__ void __launch_bounds__(kThreads, 1) int8_tcgen05_kernel(const __grid_
             break;
           }
           tc::fence_after_sync();
-          const uint32_t a_lo = field0 + s * (L::kStageBytes >> 4), b_lo = a_lo + (L::kABytes >> 4), bar = empty0 + s * 8;
-          if (++s == STAGES) {
+          const uint32_t a_lo = field0 + s * (stage_bytes >> 4), b_lo = a_lo + (a_bytes >> 4), bar = empty0 + s * 8;
+          if (++s == (uint32_t)STAGES) {
             s = 0;
             ph ^= 1;
           }
           // a look at the next stage, answered while the MMAs are being issued
           const uint32_t next = tc::mbar_test_addr(full0 + s * 8, ph);
+#pragma unroll 1
+          for (int g = 0; g < p.group; ++g) {
+            const uint32_t a_g = a_lo + g * a_block, b_g = b_lo + g * b_block;
 #pragma unroll
-          for (int h = 0; h < MH; ++h) {
+            for (int h = 0; h < MH; ++h) {
 #pragma unroll
-            for (int k = 0; k < kBK / 32; ++k) {
-              // 32 bytes of K per instruction: advance both start addresses by 32 >> 4 = 2; the second
-              // 128-row half of the A stage starts 128 * 128 bytes further (>> 4 = 1024)
-              tc::mma_i8_if(leader, d_tmem + h * BN, tc::smem_desc_from_words(a_lo + h * (kBM * kBK / 16) + 2 * k, desc_hi),
-                            tc::smem_desc_from_words(b_lo + 2 * k, desc_hi), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+              for (int k = 0; k < kBK / 32; ++k) {
+                // 32 bytes of K per instruction: advance both start addresses by 32 >> 4 = 2; the second
+                // 128-row half of the A stage starts 128 * 128 bytes further (>> 4 = 1024)
+                tc::mma_i8_if(leader, d_tmem + h * acc_cols, tc::smem_desc_from_words(a_g + h * (kBM * kBK / 16) + 2 * k, desc_hi),
+                              tc::smem_desc_from_words(b_g + 2 * k, desc_hi), idesc, (kb > 0 || g > 0 || k > 0) ? 1u : 0u);
+              }
             }
           }
           tc::mma_commit_if(leader, bar);
@@ -396,11 +404,12 @@ __global__ void __launch_bounds__(kThreads, 1) int8_tcgen05_kernel(const __grid_
     for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++local) {
       const int m0 = (tile % p.m_tiles) * (MH * kBM);
       const int n0 = (tile / p.m_tiles) * BN;
-      const uint32_t buf = (uint32_t)local % NBUF;
-      const uint32_t use = (uint32_t)local / NBUF;
-      float *v_wscale = s_vec + (local & 1) * 3 * BN;
-      float *v_bias = v_wscale + BN;
-      int32_t *v_rowsum = reinterpret_cast<int32_t *>(v_bias + BN);
+      const uint32_t buf = NBUF == 2 ? (uint32_t)local & 1u : 0u;
+      const uint32_t use = NBUF == 2 ? (uint32_t)local >> 1 : (uint32_t)local;
+      float *v_wscale = s_vec + (local & 1) * 3 * kMaxBN;
+      float *v_bias = v_wscale + kMaxBN;
+      int32_t *v_rowsum = reinterpret_cast<int32_t *>(v_bias + kMaxBN);
+      const int n_end = min(p.N, n0 + BN);               // the 32-column chunks may reach past a tile's width
       if (EPI != kEpiS32) {
         for (int j = et; j < BN; j += kEpiWarps * 32) {
           const int n = n0 + j;
@@ -430,37 +439,38 @@ __global__ void __launch_bounds__(kThreads, 1) int8_tcgen05_kernel(const __grid_
           s_m = p.src_scale[0];
           if (p.src_zp) zp_m = p.src_zp[0];
         }
-        const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + (buf * MH + h) * BN;
+        const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + (buf * MH + h) * acc_cols;
 #pragma unroll 1
         for (int c = parity * 32; c < BN; c += 64) {
           uint32_t r[32];
           tc::tmem_ld_32x32b_x32(t_row + c, r);
           tc::tmem_ld_wait();
           const int nb = n0 + c;
-          if (row_ok && nb < p.N) {
+          if (row_ok && nb < n_end) {
             if (EPI == kEpiS32) {
               int32_t *dst = reinterpret_cast<int32_t *>(p.y) + (size_t)m * p.N + nb;
-              if (nb + 32 <= p.N && (p.N & 3) == 0) {
 #pragma unroll
-                for (int j = 0; j < 32; j += 4)
+              for (int j = 0; j < 32; j += 4) {
+                if ((p.N & 3) == 0 && nb + j + 4 <= n_end) {
                   *reinterpret_cast<uint4 *>(dst + j) = make_uint4(r[j], r[j + 1], r[j + 2], r[j + 3]);
-              } else {
+                } else {
 #pragma unroll
-                for (int j = 0; j < 32; ++j)
-                  if (nb + j < p.N) dst[j] = (int32_t)r[j];
+                  for (int e = 0; e < 4; ++e)
+                    if (nb + j + e < n_end) dst[j + e] = (int32_t)r[j + e];
+                }
               }
             } else if (EPI == kEpiStatic) {
-              finish_chunk_static(p, r, s_m, zp_m, v_wscale + c, v_bias + c, v_rowsum + c, out_quant, m, nb);
+              finish_chunk_static(p, r, s_m, zp_m, v_wscale + c, v_bias + c, v_rowsum + c, out_quant, m, nb, n_end);
             } else {
               const float *ws = v_wscale + c, *bs = v_bias + c;
               const int32_t *rs = v_rowsum + c;
               switch (unary) {
-                case ZT_POST_NONE: finish_chunk<ZT_POST_NONE>(p, r, s_m, zp_m, ws, bs, rs, m, nb); break;
-                case ZT_POST_RELU: finish_chunk<ZT_POST_RELU>(p, r, s_m, zp_m, ws, bs, rs, m, nb); break;
-                case ZT_POST_SILU: finish_chunk<ZT_POST_SILU>(p, r, s_m, zp_m, ws, bs, rs, m, nb); break;
-                case ZT_POST_GELU_TANH: finish_chunk<ZT_POST_GELU_TANH>(p, r, s_m, zp_m, ws, bs, rs, m, nb); break;
-                case ZT_POST_GELU_ERF: finish_chunk<ZT_POST_GELU_ERF>(p, r, s_m, zp_m, ws, bs, rs, m, nb); break;
-                default: finish_chunk<-1>(p, r, s_m, zp_m, ws, bs, rs, m, nb); break;
+                case ZT_POST_NONE: finish_chunk<ZT_POST_NONE>(p, r, s_m, zp_m, ws, bs, rs, m, nb, n_end); break;
+                case ZT_POST_RELU: finish_chunk<ZT_POST_RELU>(p, r, s_m, zp_m, ws, bs, rs, m, nb, n_end); break;
+                case ZT_POST_SILU: finish_chunk<ZT_POST_SILU>(p, r, s_m, zp_m, ws, bs, rs, m, nb, n_end); break;
+                case ZT_POST_GELU_TANH: finish_chunk<ZT_POST_GELU_TANH>(p, r, s_m, zp_m, ws, bs, rs, m, nb, n_end); break;
+                case ZT_POST_GELU_ERF: finish_chunk<ZT_POST_GELU_ERF>(p, r, s_m, zp_m, ws, bs, rs, m, nb, n_end); break;
+                default: finish_chunk<-1>(p, r, s_m, zp_m, ws, bs, rs, m, nb, n_end); break;
               }
             }
           }
@@ -482,44 +492,10 @@ __global__ void __launch_bounds__(kThreads, 1) int8_tcgen05_kernel(const __grid_
   }
 }
 
-// ---- launch of one configuration ---------------------------------------------------------------------
-template <int MH, int BN, int STAGES, int NBUF, int EPI, bool A_SIGNED>
-int launch_cfg(const CUtensorMap &ta, const CUtensorMap &tb, const TcParams &p, cudaStream_t st) {
-  using L = SmemLayout<MH, BN, STAGES>;
-  static_assert(L::kTotal <= 227 * 1024, "stage ring exceeds shared memory");
-  auto kern = int8_tcgen05_kernel<MH, BN, STAGES, NBUF, EPI, A_SIGNED>;
-  static PerDeviceOnce configured;
-  if (int rc_cfg = allow_dynamic_smem(configured, kern, L::kTotal)) return rc_cfg;
-  TcParams q = p;
-  q.m_tiles = ceil_div(p.M, MH * kBM);
-  q.n_tiles = ceil_div(p.N, BN);
-  const int tiles = q.m_tiles * q.n_tiles;
-  const int sms = sm_count();
-  dim3 grid((unsigned)(tiles < sms ? tiles : sms));
-  ZT_CUDA_OK(launch_overlapped(kern, grid, dim3(kThreads), (size_t)L::kTotal, st, ta, tb, q));
-  return launch_status("int8_tcgen05_kernel");
-}
-
-template <int MH, int BN, int STAGES, int NBUF>
-int launch_bn(const CUtensorMap &ta, const CUtensorMap &tb, const TcParams &p, int epi, bool a_signed, cudaStream_t st) {
-  if (epi == kEpiS32)
-    return a_signed ? launch_cfg<MH, BN, STAGES, NBUF, kEpiS32, true>(ta, tb, p, st)
-                    : launch_cfg<MH, BN, STAGES, NBUF, kEpiS32, false>(ta, tb, p, st);
-  if (epi == kEpiStatic)
-    return a_signed ? launch_cfg<MH, BN, STAGES, NBUF, kEpiStatic, true>(ta, tb, p, st)
-                    : launch_cfg<MH, BN, STAGES, NBUF, kEpiStatic, false>(ta, tb, p, st);
-  return a_signed ? launch_cfg<MH, BN, STAGES, NBUF, kEpiLinear, true>(ta, tb, p, st)
-                  : launch_cfg<MH, BN, STAGES, NBUF, kEpiLinear, false>(ta, tb, p, st);
-}
-
 // CTA pairs (tcgen05.mma.cta_group::2): 512 x bn tiles, each CTA loads half of every weight block.  Linear
 // epilogue only.  Own translation unit (int8_tcgen05_pair.cu).
 bool int8_pair_supported(int64_t M, int bn);
 int launch_pair(int bn, const Int8GemmArgs &a, const TcParams &p, bool a_signed, cudaStream_t st);
-
-// 256-row tiles, instantiated in their own translation unit.
-int launch_mh2(int bn, const CUtensorMap &ta, const CUtensorMap &tb, const TcParams &p, int epi, bool a_signed,
-               cudaStream_t st);
 
 }  // namespace i8tc
 }  // namespace zt

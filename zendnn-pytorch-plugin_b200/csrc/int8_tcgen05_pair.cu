@@ -280,12 +280,12 @@ __global__ void __launch_bounds__(kThreads, 1) int8_tcgen05_pair_kernel(const __
             const float *ws = v_wscale + c, *bs = v_bias + c;
             const int32_t *rs = v_rowsum + c;
             switch (unary) {
-              case ZT_POST_NONE: finish_chunk<ZT_POST_NONE>(p, r, s_m, zp_m, ws, bs, rs, m, nb); break;
-              case ZT_POST_RELU: finish_chunk<ZT_POST_RELU>(p, r, s_m, zp_m, ws, bs, rs, m, nb); break;
-              case ZT_POST_SILU: finish_chunk<ZT_POST_SILU>(p, r, s_m, zp_m, ws, bs, rs, m, nb); break;
-              case ZT_POST_GELU_TANH: finish_chunk<ZT_POST_GELU_TANH>(p, r, s_m, zp_m, ws, bs, rs, m, nb); break;
-              case ZT_POST_GELU_ERF: finish_chunk<ZT_POST_GELU_ERF>(p, r, s_m, zp_m, ws, bs, rs, m, nb); break;
-              default: finish_chunk<-1>(p, r, s_m, zp_m, ws, bs, rs, m, nb); break;
+              case ZT_POST_NONE: finish_chunk<ZT_POST_NONE>(p, r, s_m, zp_m, ws, bs, rs, m, nb, min(p.N, n0 + BN)); break;
+              case ZT_POST_RELU: finish_chunk<ZT_POST_RELU>(p, r, s_m, zp_m, ws, bs, rs, m, nb, min(p.N, n0 + BN)); break;
+              case ZT_POST_SILU: finish_chunk<ZT_POST_SILU>(p, r, s_m, zp_m, ws, bs, rs, m, nb, min(p.N, n0 + BN)); break;
+              case ZT_POST_GELU_TANH: finish_chunk<ZT_POST_GELU_TANH>(p, r, s_m, zp_m, ws, bs, rs, m, nb, min(p.N, n0 + BN)); break;
+              case ZT_POST_GELU_ERF: finish_chunk<ZT_POST_GELU_ERF>(p, r, s_m, zp_m, ws, bs, rs, m, nb, min(p.N, n0 + BN)); break;
+              default: finish_chunk<-1>(p, r, s_m, zp_m, ws, bs, rs, m, nb, min(p.N, n0 + BN)); break;
             }
           }
           __syncwarp();
