@@ -1092,6 +1092,8 @@ int woq_tcgen05_launch(const zt_woq_linear_args_t &a, cudaStream_t st) {
   p.post = to_dev(a.post);
   p.status = device_status_ptr();
   const int hint = (a.algo >> 8) & 0xffff;
+  ZT_REQUIRE(hint == 0 || hint == 32 || hint == 64 || hint == 128 || hint == 256, ZT_UNSUPPORTED,
+             "zt_woq_linear: unsupported token-tile width %d for the tcgen05 kernel", hint);
   const bool may_split = hint == 0 && !(a.algo & ZT_ALGO_SINGLE_ISSUER) && a.workspace != nullptr;
   DensePlan d = dense_plan(a.M, a.N, a.K, hint, may_split);
   if (d.split && a.workspace_bytes < ZT_WOQ_COUNTER_BYTES + split_bytes(d)) d = dense_plan(a.M, a.N, a.K, hint, false);
