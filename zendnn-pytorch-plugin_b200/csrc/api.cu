@@ -232,8 +232,8 @@ extern "C" int zt_selftest_expire_wait(void *stream) {
 }
 
 // ---- weight-only int4 ---------------------------------------------------------------------------
-extern "C" size_t zt_woq_linear_workspace_bytes(int64_t M, int64_t N, int64_t K) {
-  if (M <= 0 || N <= 0 || K <= 0) return ZT_WOQ_COUNTER_BYTES;
+namespace {
+size_t woq_workspace_bytes(int64_t M, int64_t N, int64_t K) {
   const size_t a = woq_skinny_plan(M, N, K).partial_bytes;
   const size_t b = woq_stream_plan(M < 16 ? M : 16, N, K).partial_bytes;
   const size_t c = woq_streamk_workspace_bytes();
@@ -241,6 +241,23 @@ extern "C" size_t zt_woq_linear_workspace_bytes(int64_t M, int64_t N, int64_t K)
   size_t m = a > b ? a : b;
   m = m > c ? m : c;
   return ZT_WOQ_COUNTER_BYTES + (m > d ? m : d);
+}
+}  // namespace
+
+extern "C" size_t zt_woq_linear_workspace_bytes(int64_t M, int64_t N, int64_t K) {
+  if (M <= 0 || N <= 0 || K <= 0) return ZT_WOQ_COUNTER_BYTES;
+  // Every call of the operator asks for this, and the kernels' plans behind it are some dozens of 64-bit divisions: the
+  // answer is a function of the sizes and the SM count alone and is kept for the last sizes of each thread.
+  struct Entry {
+    int64_t m, n, k;
+    int sms;
+    size_t bytes;
+  };
+  thread_local Entry table[64] = {};
+  const int sms = sm_count();
+  Entry &e = table[((uint64_t)M * 31 + (uint64_t)N * 7 + (uint64_t)K / 8) % 64];
+  if (e.m != M || e.n != N || e.k != K || e.sms != sms) e = Entry{M, N, K, sms, woq_workspace_bytes(M, N, K)};
+  return e.bytes;
 }
 
 extern "C" int zt_woq_linear(const zt_woq_linear_args_t *a, void *stream) {

@@ -1,7 +1,8 @@
 // Per-token dynamic quantisation of activations: the first phase of zentorch_dynamic_qlinear.
 //
-// One CTA per row.  The row is read once into registers (up to 32 values per thread; longer rows
-// re-read the tail, which then comes from L2), reduced to its absolute maximum (s8) or min/max (u8)
+// One CTA per row, of 256 threads, or 1024 where the rows are fewer than the SMs: then a row's latency is the kernel's
+// (M = 1, K = 8192: a thread's 32 divisions against 8).  The row is read once into registers (up to 32 values per
+// thread; longer rows re-read the tail, which then comes from L2), reduced to its absolute maximum (s8) or min/max (u8)
 // with warp shuffles, and written back as 8-bit values with 8-byte stores.  The scale uses IEEE
 // division and the quantised value round-half-even, so the bytes equal those of the CPU formula
 //   s = max(absmax, 1e-12) / 127,   q = clamp(rint(x / s), -128, 127).
@@ -16,7 +17,7 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kVec = 8;        // elements per thread per chunk
-constexpr int kCached = 4;     // chunks kept in registers
+constexpr int kWideThreads = 1024;
 
 __device__ __forceinline__ void load8(const void *x, int dtype, int64_t off, float (&v)[8]) {
   if (dtype == ZT_BF16) {
@@ -42,6 +43,7 @@ __device__ __forceinline__ void load8(const void *x, int dtype, int64_t off, flo
 __device__ __forceinline__ float nan_max(float a, float b) { return (a != a) ? a : (b != b) ? b : fmaxf(a, b); }
 __device__ __forceinline__ float nan_min(float a, float b) { return (a != a) ? a : (b != b) ? b : fminf(a, b); }
 
+template <int THREADS>
 __device__ __forceinline__ void block_reduce_max_min(float &hi, float &lo, bool saw_nan, float *scratch) {
   if (saw_nan) hi = lo = __int_as_float(0x7fc00000);
 #pragma unroll
@@ -49,17 +51,27 @@ __device__ __forceinline__ void block_reduce_max_min(float &hi, float &lo, bool 
     hi = nan_max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
     lo = nan_min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
   }
-  constexpr int kWarps = kThreads / 32;
+  constexpr int kWarps = THREADS / 32;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (lane == 0) {
     scratch[warp] = hi;
     scratch[kWarps + warp] = lo;
   }
   __syncthreads();
+  if (kWarps == 32) {          // one result per lane: another shuffle reduction instead of 32 serial steps
+    hi = scratch[lane];
+    lo = scratch[kWarps + lane];
 #pragma unroll
-  for (int w = 0; w < kWarps; ++w) {
-    hi = nan_max(hi, scratch[w]);
-    lo = nan_min(lo, scratch[kWarps + w]);
+    for (int o = 16; o > 0; o >>= 1) {
+      hi = nan_max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+      lo = nan_min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+    }
+  } else {
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) {
+      hi = nan_max(hi, scratch[w]);
+      lo = nan_min(lo, scratch[kWarps + w]);
+    }
   }
 }
 
@@ -88,11 +100,12 @@ __device__ __forceinline__ uint32_t quant_one(float x, float s, float zp) {
 }
 
 // Vector path: K % 8 == 0 and 16-byte aligned rows.
-template <bool U8>
-__global__ void __launch_bounds__(kThreads) dynquant_vec_kernel(const void *__restrict__ x, int x_dtype, int64_t K,
+template <bool U8, int THREADS>
+__global__ void __launch_bounds__(THREADS) dynquant_vec_kernel(const void *__restrict__ x, int x_dtype, int64_t K,
                                                                 uint8_t *__restrict__ q, float *__restrict__ scales,
                                                                 int32_t *__restrict__ zps) {
-  __shared__ float scratch[16];
+  constexpr int kCached = THREADS == kWideThreads ? 2 : 4;   // chunks kept in registers
+  __shared__ float scratch[2 * THREADS / 32];
   // programmatic dependent launch: let the GEMM that follows start its prologue and weight prefetch now;
   // wait for the kernel before this one (it may still read the buffers written here) before any access
   grid_launch_dependents();
@@ -105,7 +118,7 @@ __global__ void __launch_bounds__(kThreads) dynquant_vec_kernel(const void *__re
   bool saw_nan = false;
 #pragma unroll
   for (int c = 0; c < kCached; ++c) {
-    const int64_t ch = (int64_t)c * kThreads + threadIdx.x;
+    const int64_t ch = (int64_t)c * THREADS + threadIdx.x;
     if (ch < chunks) {
       load8(x, x_dtype, base + ch * kVec, v[c]);
 #pragma unroll
@@ -120,7 +133,7 @@ __global__ void __launch_bounds__(kThreads) dynquant_vec_kernel(const void *__re
       }
     }
   }
-  for (int64_t ch = (int64_t)kCached * kThreads + threadIdx.x; ch < chunks; ch += kThreads) {
+  for (int64_t ch = (int64_t)kCached * THREADS + threadIdx.x; ch < chunks; ch += THREADS) {
     float t[8];
     load8(x, x_dtype, base + ch * kVec, t);
 #pragma unroll
@@ -134,7 +147,7 @@ __global__ void __launch_bounds__(kThreads) dynquant_vec_kernel(const void *__re
       }
     }
   }
-  block_reduce_max_min(hi, lo, saw_nan, scratch);
+  block_reduce_max_min<THREADS>(hi, lo, saw_nan, scratch);
   float s, zp;
   row_scale<U8>(hi, lo, s, zp);
   if (threadIdx.x == 0) {
@@ -152,10 +165,10 @@ __global__ void __launch_bounds__(kThreads) dynquant_vec_kernel(const void *__re
   };
 #pragma unroll
   for (int c = 0; c < kCached; ++c) {
-    const int64_t ch = (int64_t)c * kThreads + threadIdx.x;
+    const int64_t ch = (int64_t)c * THREADS + threadIdx.x;
     if (ch < chunks) emit(v[c], ch);
   }
-  for (int64_t ch = (int64_t)kCached * kThreads + threadIdx.x; ch < chunks; ch += kThreads) {
+  for (int64_t ch = (int64_t)kCached * THREADS + threadIdx.x; ch < chunks; ch += THREADS) {
     float t[8];
     load8(x, x_dtype, base + ch * kVec, t);
     emit(t, ch);
@@ -184,7 +197,7 @@ __global__ void __launch_bounds__(kThreads) dynquant_scalar_kernel(const void *_
       hi = fmaxf(hi, fabsf(t));
     }
   }
-  block_reduce_max_min(hi, lo, saw_nan, scratch);
+  block_reduce_max_min<kThreads>(hi, lo, saw_nan, scratch);
   float s, zp;
   row_scale<U8>(hi, lo, s, zp);
   if (threadIdx.x == 0) {
@@ -266,10 +279,11 @@ int dynamic_quantize_launch(const void *x, int x_dtype, int64_t M, int64_t K, in
   uint8_t *qq = reinterpret_cast<uint8_t *>(q);
   const dim3 grid((unsigned)M);
   if (vec) {
-    if (u8)
-      ZT_CUDA_OK(launch_overlapped(dynquant_vec_kernel<true>, dim3(grid), dim3(kThreads), (size_t)0, st, x, x_dtype, K, qq, scales, zps));
-    else
-      ZT_CUDA_OK(launch_overlapped(dynquant_vec_kernel<false>, dim3(grid), dim3(kThreads), (size_t)0, st, x, x_dtype, K, qq, scales, zps));
+    // few rows: one wide CTA per row and SM (a row of at least two chunks per thread of the narrow form)
+    const bool wide = M <= sm_count() && K >= 2 * kThreads * kVec;
+    auto kern = wide ? (u8 ? dynquant_vec_kernel<true, kWideThreads> : dynquant_vec_kernel<false, kWideThreads>)
+                     : (u8 ? dynquant_vec_kernel<true, kThreads> : dynquant_vec_kernel<false, kThreads>);
+    ZT_CUDA_OK(launch_overlapped(kern, grid, dim3(wide ? kWideThreads : kThreads), (size_t)0, st, x, x_dtype, K, qq, scales, zps));
   } else {
     if (u8)
       ZT_CUDA_OK(launch_overlapped(dynquant_scalar_kernel<true>, dim3(grid), dim3(kThreads), (size_t)0, st, x, x_dtype, K, qq, scales, zps));
