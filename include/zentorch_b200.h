@@ -76,12 +76,14 @@ typedef enum {
   ZT_ALGO_SKINNY = 2,  /* small M, HBM-bound streaming kernel */
   ZT_ALGO_TCGEN05 = 3  /* large M, tcgen05 tensor cores with TMEM accumulators */
 } zt_algo_t;
-/* An `algo` argument may carry a tile-width hint for the tcgen05 kernels in bits 8..23 (0 = choose);
- * tests and benchmarks use it to exercise every compiled tile shape. */
+/* An `algo` argument may carry a tile hint for the tcgen05 kernels in bits 8..23 (0 = choose); tests and benchmarks use it to
+ * reach shapes that the choice does not take.  Weight-only: the kernel for tiles of up to 32, 64, 128 or 192 (hint 256) rows,
+ * without K slices.  int8: the tile's width, a multiple of 16 up to 256; + 1000 for tiles of 256 rows; + 2000 for CTA pairs. */
 #define ZT_ALGO_WITH_TILE(algo, tile_n) ((int32_t)(algo) | ((int32_t)(tile_n) << 8))
-/* Bit 24: the weight-only tcgen05 kernel gives every tile of the output to one CTA, which sums all of K in order, instead of
- * sharing a tile's K between CTAs where that is faster (tests compare the two forms). */
-#define ZT_ALGO_SINGLE_ISSUER (1 << 24)
+/* Bit 24: the weight-only tcgen05 kernel sums all of K in order in one accumulator, instead of alternate blocks of K in two
+ * and slices of K on several SMs (tests compare the forms). */
+#define ZT_ALGO_ONE_ACCUMULATOR (1 << 24)
+#define ZT_ALGO_SINGLE_ISSUER ZT_ALGO_ONE_ACCUMULATOR /* its former name */
 
 ZT_API const char *zt_last_error(void);
 ZT_API const char *zt_version(void);
@@ -104,6 +106,11 @@ ZT_API int zt_selftest_expire_wait(void *stream);
  * stay zero).  Records hold 8 uint64 each; launches that no longer fit are not recorded.  Pass NULL to
  * switch it off (the default). */
 ZT_API int zt_debug_set_timeline(void *device_buffer, size_t bytes);
+
+/* How the weight-only tcgen05 kernel divides an [M, K] x [K, N] call on the current device: {rows that its kernel's tiles can
+ * hold, row tiles, rows per tile, K slices per tile, accumulators per slice}.  `fp32_conversion`: fp32 scales with zero points.
+ * Tests check with it that their shapes reach what they mean to. */
+ZT_API int zt_debug_woq_plan(int64_t M, int64_t N, int64_t K, int32_t fp32_conversion, int32_t plan[5]);
 
 /* ---------------------------------------------------------------------------------------------
  * Weight-only int4 linear.   zentorch_woq_linear_impl, src/cpu/cpp/WOQ_Linear.cpp:14-176, and the

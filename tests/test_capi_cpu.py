@@ -194,3 +194,24 @@ def test_static_qlinear_validation_schemas_and_meta(zt):
         ops.zentorch_qlinear(torch.zeros(2, 8), torch.zeros(4, 8, dtype=torch.int8), torch.ones(1),
                              torch.zeros(1, dtype=torch.int32), torch.ones(4), torch.zeros(4, dtype=torch.int32),
                              None, None, None)
+
+
+def test_woq_plan_keeps_sums_short(zt):
+    """The tensor-core weight-only kernel's plan, for 148 SMs: K is divided among at least as many fp32 sums as two accumulators
+    (up to 128 rows) and as many equal slices as fit the SMs at once (up to 256 rows) give; slices are of whole chunks."""
+    from zentorch_b200 import _capi
+    if _capi.lib().zt_device_supported():
+        pytest.skip("the numbers are for 148 SMs")
+    for m in (1, 17, 32, 33, 64, 65, 128, 129, 192, 193, 256, 257, 384, 1000, 2048):
+        for n in (8, 136, 1000, 1024, 4096, 5003, 8192, 14336, 28672):
+            for k in (64, 192, 512, 2816, 4096, 8192, 8256, 14336):
+                for fp32_conversion in (False, True):
+                    cap, m_tiles, bt, slices, accs = _capi.woq_plan(m, n, k, fp32_conversion)
+                    n_tiles, chunks = -(-n // 128), -(-k // 256)
+                    assert bt <= cap and bt % 16 == 0 and (m_tiles - 1) * bt < m <= m_tiles * bt
+                    assert 1 <= slices <= min(32, chunks) and accs in (1, 2) and (accs == 1 or cap <= 128)
+                    equal = [d for d in range(1, 33) if k % (256 * d) == 0 and n_tiles * d <= 148]
+                    wanted = (2 if m <= 128 else 1) * max(equal + [1]) if m <= 256 else 1
+                    assert slices * accs >= wanted, (m, n, k, slices, accs, wanted)
+                    if slices > 1:
+                        assert _capi.lib().zt_woq_linear_workspace_bytes(m, n, k) >= 16384 + slices * m * -(-n // 4) * 16

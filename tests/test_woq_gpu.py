@@ -175,7 +175,7 @@ def test_post_ops(capi, name, algo_name):
     assert_close_bf16(y, O.woq_linear(x, packed.t(), s, None, b, ops, bufs), what=name)
 
 
-# ---- tensor-core kernel (M > 16): every token-tile width, ragged M / N, both quantisation forms ------------
+# ---- tensor-core kernel (M > 16): every instantiation (a hint chooses it), ragged M / N, both quantisation forms ------------
 @pytest.mark.parametrize("tile", [0, 32, 64, 128, 256])
 @pytest.mark.parametrize("asym,scale_dtype", [(False, torch.float32), (False, torch.bfloat16), (True, torch.float32),
                                               (True, torch.bfloat16)])
@@ -183,7 +183,7 @@ def test_tcgen05_kernel(capi, tile, asym, scale_dtype):
     # K = 128, 320, 448: packed-weight chunks of four k-blocks that end in a partial chunk
     for (m, k, n, gs) in ((17, 256, 128, 128), (100, 512, 200, 64), (300, 1024, 136, 128), (64, 128, 8, 32),
                           (257, 2048, 384, 2048), (40, 320, 72, 32), (129, 448, 260, 64),
-                          (64, 1024, 256, 128), (200, 2048, 136, 64)):   # few tiles, long K: split over K when tile == 0
+                          (64, 1024, 256, 128), (200, 2048, 136, 64)):   # few tiles: K in slices when tile == 0
         x, q, s, z, b = make_woq_case(m, k, n, gs, seed=m + n, asym=asym, scale_dtype=scale_dtype)
         algo = capi.ZT_ALGO_TCGEN05 | (tile << 8)
         y, packed = _run(capi, x, q, s, z, b, algo)
@@ -194,47 +194,79 @@ def test_tcgen05_kernel(capi, tile, asym, scale_dtype):
         assert (y.float() - ref.float()).abs().max() <= tight * max(1.0, float(ref.float().abs().max())), (m, k, n)
 
 
-@pytest.mark.parametrize("m,k,n", [(40, 128, 136), (33, 192, 128), (64, 4096, 256), (128, 1024, 384), (300, 2048, 200)])
-def test_tcgen05_one_and_two_issuers_agree(capi, m, k, n):
-    """The kernel's default form has two MMA issuers, each summing every other k-block into an accumulator of
-    its own (the epilogue adds them); the one-issuer form sums all k-blocks in order.  Both against the oracle,
-    and against each other to fp32 summation-order noise (K = 192: three k-blocks, the issuers swap parity from
-    tile to tile)."""
+@pytest.mark.parametrize("m,k,n", [(40, 128, 136), (33, 192, 128), (17, 64, 136), (64, 4096, 256), (128, 1024, 384), (300, 2048, 200),
+                                   (30, 512, 19100), (60, 512, 19100), (128, 512, 19100)])
+def test_tcgen05_accumulators_agree(capi, m, k, n):
+    """Up to 128 rows the kernel sums alternate blocks of 64 k in two accumulators, which the epilogue adds; bit 24 makes it sum all of
+    K in one, in order.  Both against the oracle, and against each other to fp32 summation-order noise (K = 64: the second
+    accumulator has nothing in it; N = 19100: a CTA has two tiles and the accumulators change hands, in two sets or in one)."""
     x, q, s, z, b = make_woq_case(m, k, n, 64, seed=k + n)
     y2, packed = _run(capi, x, q, s, None, b, capi.ZT_ALGO_TCGEN05)
-    y1, _ = _run(capi, x, q, s, None, b, capi.ZT_ALGO_TCGEN05 | capi.ZT_ALGO_SINGLE_ISSUER)
+    y1, _ = _run(capi, x, q, s, None, b, capi.ZT_ALGO_TCGEN05 | capi.ZT_ALGO_ONE_ACCUMULATOR)
     ref = O.woq_linear(x, packed.t(), s, None, b)
-    assert_close_bf16(y2, ref, what=f"two issuers {m}x{k}x{n}")
-    assert_close_bf16(y1, ref, what=f"one issuer {m}x{k}x{n}")
+    assert_close_bf16(y2, ref, what=f"two accumulators {m}x{k}x{n}")
+    assert_close_bf16(y1, ref, what=f"one accumulator {m}x{k}x{n}")
     # the two forms round one fp32 sum differently: at most one bf16 ulp apart, and mostly equal
     d = (y1.float() - y2.float()).abs()
     assert float(d.max()) <= 2 ** -7 * max(1.0, float(ref.float().abs().max()))
     assert float((d == 0).float().mean()) > 0.9
+    assert (capi.woq_plan(m, n, k)[4] == 2) == (m <= 128)
+    if m <= 128 and k >= 4096:
+        assert not torch.equal(y1, y2)          # the comparison is of two different sums
 
 
-@pytest.mark.parametrize("m,k,n,gs,asym,scale_dtype", [
-    (20, 14336, 136, 128, False, torch.float32),     # two tiles, sixteen CTAs each; last column tile eight wide
-    (17, 8256, 130, 64, True, torch.bfloat16),       # K = 32 x 256 + 64: void stage; group of 64; odd row pitch of the scales
-    (129, 14400, 132, 32, False, torch.bfloat16),    # two row tiles, groups of 32
-    (64, 12288, 257, 12288, True, torch.float32),    # one group, odd number of columns
-    (190, 16384, 128, 256, False, torch.float32)])   # one 192-token tile
-def test_tcgen05_shared_tiles(capi, m, k, n, gs, asym, scale_dtype):
-    """Few tiles with a long K: their chunks are dealt to many CTAs and the pieces added by the last to arrive.
+@pytest.mark.parametrize("m,k,n,limit", [(32, 4096, 14336, 2.4e-6), (128, 8192, 8192, 2.4e-6), (20, 14336, 136, 3e-7), (64, 512, 4096, 1.4e-7)])
+def test_tcgen05_accumulation_error(capi, m, k, n, limit):
+    """The error of the fp32 sums, seen through a bf16 result by subtracting the exact value (in two bf16 parts, as operands of
+    two additions) before the rounding.  The tensor core truncates what it adds, so the error grows with the length of a sum;
+    measured relative to the result's root mean square, in one sum / as divided now: 3.5e-6 / 1.6e-6, 7.7e-6 / 1.6e-6,
+    6.4e-7 / 1.9e-7, 3.2e-7 / 8.7e-8.  bf16 scales: the dequantised weight is exactly bf16(q * s)."""
+    g = torch.Generator(device="cuda").manual_seed(3)
+    x = torch.randn(m, k, generator=g, device="cuda").to(torch.bfloat16)
+    q = torch.randint(-8, 8, (n, k), generator=g, device="cuda", dtype=torch.int8)
+    s = (torch.rand(k // 128, n, generator=g, device="cuda") * 4e-3 + 1e-3).to(torch.bfloat16)
+    w = (q.float().view(n, k // 128, 128) * s.float().t().unsqueeze(2)).view(n, k).to(torch.bfloat16)
+    exact = x.double() @ w.double().t()
+    hi = exact.to(torch.bfloat16)
+    lo = (exact - hi.double()).to(torch.bfloat16)
+    y = capi.woq_linear(x, capi.woq_repack_weight(q), s, None, None, [capi.ZT_POST_ADD, capi.ZT_POST_ADD], [-hi, -lo],
+                        algo=capi.ZT_ALGO_TCGEN05)
+    err = y.double() - (exact - hi.double() - lo.double())
+    assert float(err.pow(2).mean().sqrt() / exact.pow(2).mean().sqrt()) <= limit
+
+
+@pytest.mark.parametrize("m,k,n,gs,asym,scale_dtype,cap", [
+    (20, 14336, 136, 128, False, torch.float32, 32),     # two column tiles, the last eight wide
+    (17, 8256, 130, 64, True, torch.bfloat16, 32),       # K = 32 x 256 + 64: slices of unequal length, the last with a void stage; odd row pitch
+    (24, 2816, 640, 64, True, torch.float32, 32),        # eleven chunks; scales and zero points of four groups a chunk
+    (50, 4416, 520, 64, False, torch.float32, 64),       # the last slice has 64 k in its last chunk
+    (60, 4096, 1024, 32, True, torch.bfloat16, 64),      # eight groups a chunk
+    (64, 12288, 257, 12288, True, torch.float32, 64),    # one group, odd number of columns
+    (120, 14400, 132, 32, False, torch.bfloat16, 128),   # groups of 32, scales from global memory
+    (128, 8256, 1000, 32, True, torch.float32, 128),     # eight groups a chunk, the largest slot
+    (250, 14336, 4096, 128, True, torch.float32, 128),   # two row tiles
+    (150, 14336, 1280, 128, True, torch.bfloat16, 192),
+    (150, 14336, 1281, 64, False, torch.float32, 192),   # scales from global memory
+    (700, 14336, 1000, 64, False, torch.float32, 192)])  # more than 256 rows: cut for speed alone
+def test_tcgen05_k_slices(capi, m, k, n, gs, asym, scale_dtype, cap):
+    """Few tiles with a long K: slices of K on several SMs, whose sums a second kernel adds.
     Against the oracle; against the form in which one CTA sums a tile (bit 24; the two round one fp32 sum
     differently, so one bf16 ulp); twice the same bits; with a post-op chain that reads two operands."""
+    plan = capi.woq_plan(m, n, k, asym and scale_dtype == torch.float32)
+    assert plan[0] == cap and plan[3] > 1, plan
     x, q, s, z, b = make_woq_case(m, k, n, gs, seed=m + k, asym=asym, scale_dtype=scale_dtype)
     y, packed = _run(capi, x, q, s, z, b, capi.ZT_ALGO_TCGEN05)
-    assert_close_bf16(y, O.woq_linear(x, packed.t(), s, z, b), what=f"shared tiles {m}x{k}x{n}")
+    assert_close_bf16(y, O.woq_linear(x, packed.t(), s, z, b), what=f"K slices {m}x{k}x{n}")
     again, _ = _run(capi, x, q, s, z, b, capi.ZT_ALGO_TCGEN05)
     assert torch.equal(y, again)
-    one, _ = _run(capi, x, q, s, z, b, capi.ZT_ALGO_TCGEN05 | capi.ZT_ALGO_SINGLE_ISSUER)
+    one, _ = _run(capi, x, q, s, z, b, capi.ZT_ALGO_TCGEN05 | capi.ZT_ALGO_ONE_ACCUMULATOR)
     d = (y.float() - one.float()).abs()
     assert float((d - 2 ** -7 * y.float().abs()).max()) <= 1e-4 * float(y.float().abs().max())
     ops, nbuf = POST_CASES["mul_add"]
     g = torch.Generator().manual_seed(9)
     bufs = [torch.randn(m, n, generator=g).to(torch.bfloat16) for _ in range(nbuf)]
     ym, _ = _run(capi, x, q, s, z, b, capi.ZT_ALGO_TCGEN05, ops, bufs)
-    assert_close_bf16(ym, O.woq_linear(x, packed.t(), s, z, b, ops, bufs), what=f"shared tiles, mul_add {m}x{k}x{n}")
+    assert_close_bf16(ym, O.woq_linear(x, packed.t(), s, z, b, ops, bufs), what=f"K slices, mul_add {m}x{k}x{n}")
 
 
 @pytest.mark.parametrize("name", sorted(["relu", "gelu_erf", "silu", "add", "mul_add", "add_add"]))

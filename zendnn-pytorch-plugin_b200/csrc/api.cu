@@ -208,6 +208,13 @@ extern "C" int zt_debug_set_timeline(void *device_buffer, size_t bytes) {
   return ZT_SUCCESS;
 }
 
+extern "C" int zt_debug_woq_plan(int64_t M, int64_t N, int64_t K, int32_t fp32_conversion, int32_t plan[5]) {
+  ZT_REQUIRE(M >= 1 && N >= 1 && K >= 64 && K % 64 == 0 && M <= (1 << 30) && N <= (1 << 30) && K <= (1 << 30) && plan,
+             ZT_INVALID_ARGUMENT, "zt_debug_woq_plan: not a shape of the tcgen05 kernel");
+  woq_tcgen05_plan(M, N, K, fp32_conversion != 0, plan);
+  return ZT_SUCCESS;
+}
+
 // ---- self-test of the bounded-wait path ------------------------------------------------------------
 namespace zt {
 namespace {

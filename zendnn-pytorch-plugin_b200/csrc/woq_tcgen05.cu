@@ -11,17 +11,18 @@
 //   warp 1        TMEM allocation, tcgen05.mma.kind::f16 issue (A from tensor memory, B from shared memory)
 //   warp 2        TMA producer of the packed weights in chunks of 256 k (128 rows x 128 B, 128-byte swizzle) with
 //                 their scales / zero points, several chunks ahead, never waiting for the preceding kernel
-//   warps 3..6    epilogue: tcgen05.ld (lane = output column n, register j = token), transpose through shared
-//                 memory so that stores run along n, bias + post-ops, bf16 stores
+//   warps 3..6    epilogue: tcgen05.ld (lane = output column n, register j = token), the sum of a tile's accumulators, bias +
+//                 post-ops, bf16 stores of 64 contiguous bytes per token
 //   warps 7..     conversion, teams of four warps; team t of T takes the ring positions congruent to t mod T; then,
 //                 idle, they help with the epilogue of the CTA's last tile
 //
 // What bounds it.  Converting a 128 x 64 block costs its SM about 200 cycles of the two half-rate pipes (per packed word
 // of eight weights 9 shift / permute / lop3 operations on one and 8 - 12 bf16x2 operations on the other); its MMAs take 2
-// cycles per token and at least 128.  A block takes 300 - 350 cycles up to 128 tokens (650 when the converted operand
-// went through shared memory and the issuing threads ran divergent code); M = 32 on 4096 -> 14336: 21.6 -> 13.7 us, M = 128
-// on 8192 -> 8192: 31 -> 24 us, M = 2048 on 4096 -> 14336: 259 -> 217 us (0.70 of the bf16 peak; from 128 tokens on an
-// SM pulls 35 bytes per cycle of activations and weights out of L2, which is what it can get).  What that took:
+// cycles per token and at least 128.  A block takes 300 - 350 cycles up to 64 tokens and 350 - 450 up to 128 (650 when the
+// converted operand went through shared memory and the issuing threads ran divergent code); per call, M = 32 on 4096 -> 14336:
+// 21.6 -> 15.0 us, M = 128 on 8192 -> 8192 with two operands: 39.4 -> 25.6 us, M = 2048 on 4096 -> 14336: 263 -> 219 us (0.66 of the
+// bf16 peak; from 128 tokens on an SM pulls 35 bytes per cycle of activations and weights out of L2, which is what it can
+// get).  What that took:
 //   * The converted operand lives in tensor memory: its 32 KB per block (store, then MMA read) leave the shared-memory
 //     port.
 //   * The warp index comes from a shuffle, so the compiler knows every role's control flow to be uniform across the
@@ -36,16 +37,21 @@
 // therefore waits on each of its phases in order), activation slots of XK k in shared memory (one bulk copy each; they
 // are requested long before use because a copy takes over a thousand cycles), packed chunks of 256 k.
 //
-// Work split.  The unit is a chunk (256 k of a tile).  A CTA usually takes whole tiles; where few tiles have a long K
-// ("split", see dense_plan) the chunks of all tiles are dealt to the CTAs in equal contiguous ranges.  The pieces of a
-// tile that spans CTAs go through fp32 partial sums in the workspace; the last warp to arrive (a ticket per 16 tokens x
-// 32 columns) adds them in CTA order, so results do not depend on timing.
+// Work split.  An item is a tile, or a slice of its K (whole chunks) where there are fewer tiles than SMs or a shorter sum is
+// wanted (see min_sums and dense_plan); the slices' fp32 sums go through the workspace and a second kernel adds them in order,
+// so results do not depend on timing.  Without slices the layers of few tiles leave most SMs idle: M = 17 on 4096 -> 4096 took
+// 12.8 us on 32 SMs and takes 7.9 in four slices.  The slices used to meet at the end of this kernel by tickets, which cost 5 - 10
+// us and so was hardly ever worth it.
+//
+// Sums.  The tensor core's fp32 accumulation truncates, so its error grows with the length of the sum: tiles of up to 128 rows
+// are therefore summed in two accumulators, one for each parity of the 64-k blocks, which the epilogue adds.
 //
 // Grouped mode (mixture-of-experts): the rows of X are sorted by expert, a device-side table lists the row tiles
 // {expert, first row, valid rows}, and each tile uses its expert's slice of the stacked weight and scale tensors;
 // the number of tiles is read from device memory, so no host synchronisation is needed between routing and GEMM.
 //
-// Accumulators are double buffered in tensor memory.  All waits are bounded (see tc05.cuh).
+// Accumulators are double buffered in tensor memory as far as they fit (see Accumulators).  All waits are bounded (see
+// tc05.cuh).
 //
 // Rounding.  q (an integer in [-8, 7]) is exact in bf16.  With bf16 scales q*s is one bf16x2 multiplication, i.e.
 // exactly bf16(q*s), and (q-8)*s + z one bf16x2 fma, rounded once.  With fp32 scales s is split into s_hi + s_lo
@@ -68,14 +74,12 @@ constexpr int kEpiWarps = 4;
 constexpr int kFirstTeam = 3 + kEpiWarps;   // warps 0..2: activation producer, MMA issuer, packed-weight producer
 constexpr int kPackedProducer = 2;
 constexpr int threads_for(int teams) { return 32 * (kFirstTeam + teams * kTeamWarps); }
-constexpr int kEpiRowStride = 36;   // floats; 144 bytes keeps 16-byte alignment and spreads banks
-constexpr int kEpiScratch = 16 * kEpiRowStride;   // per warp: 16 tokens x 32 columns
 constexpr int kChunkK = 256;        // k per packed chunk: one 128-byte row of nibbles
 constexpr int kChunkBytes = kBN * 128;
 // per packed chunk: up to two groups x 128 columns of fp32 scales (1 KB), then the same for zero points
 constexpr int kScaleSlotBytes = 2048;
 constexpr int kZeroSlotOffset = 1024;
-constexpr int kTickets = ZT_WOQ_COUNTER_BYTES / 4;   // one per tile, 16 tokens and 32 columns
+constexpr int kMaxSlices = 32;      // K slices of a tile
 
 // How a weight is dequantised (template parameter of the kernel).
 enum DqMode { kSymF32 = 0, kSymBf16 = 1, kAsymBf16 = 2, kAsymF32 = 3 };
@@ -83,9 +87,9 @@ enum DqMode { kSymF32 = 0, kSymBf16 = 1, kAsymBf16 = 2, kAsymF32 = 3 };
 struct TcParams {
   int M, N, K;
   int m_tiles, n_tiles, bt;   // dense mode: row tiles of bt tokens
-  int chunks;                 // per tile
+  int chunks, slices;         // per tile: chunks of K, and the slices that share them
+  int accs;                   // accumulators of a tile: 2 = one for each parity of the 64-k blocks, added by the epilogue
   int x_box, x_box2;          // rows of the activation box: the first when the tile's rows fit, else the second
-  int split;                  // chunks dealt out in equal ranges (else whole tiles)
   int gs, gs_log2;            // gs_log2 < 0: not a power of two
   const int32_t *wq;
   const void *scales;
@@ -95,8 +99,7 @@ struct TcParams {
   __nv_bfloat16 *y;
   PostOpsDev post;
   int *status;
-  float *partial;             // split: [2 * CTAs][4 quarters][NMAX / 16][16 x 32] fp32
-  unsigned int *tickets;      // split: [tiles][NMAX / 16][4], zero between launches
+  float *partial;             // slices > 1: their sums [slices][M][N rounded up to 4], which woq_slices_kernel adds
   // grouped mode (g_count != nullptr)
   const int *g_count;         // number of row tiles
   const int4 *g_tiles;        // per row tile: {expert, first row, valid rows, 0}
@@ -125,41 +128,42 @@ __device__ __forceinline__ TileInfo decode_tile(const TcParams &p, uint32_t tile
   return t;
 }
 
-// The chunks a CTA works on, tile by tile.  `total` = tiles x chunks.
+// The work of a CTA: every gridDim.x-th item, an item being a slice of K of a tile.
 struct Work {
-  uint32_t pos, end, total, chunks;
-  bool split;
-  uint32_t tile, c0, c1;   // current segment: chunks [c0, c1) of `tile`
+  uint32_t item, items, chunks, slices;
+  uint32_t tile, slice, c0, c1;   // current item: chunks [c0, c1) of `tile`
 
-  __device__ __forceinline__ Work(const TcParams &p, uint32_t n_mt) {
-    chunks = (uint32_t)p.chunks;
-    total = n_mt * (uint32_t)p.n_tiles * chunks;
-    split = p.split != 0;
-    pos = split ? first_of(blockIdx.x) : blockIdx.x * chunks;
-    end = split ? first_of(blockIdx.x + 1) : total;
-  }
-  __device__ __forceinline__ uint32_t first_of(uint32_t cta) const {
-    return (uint32_t)((uint64_t)cta * total / gridDim.x);
-  }
-  __device__ __forceinline__ uint32_t cta_of(uint32_t position) const {   // the CTA whose range holds it
-    return (uint32_t)(((uint64_t)(position + 1) * gridDim.x - 1) / total);
-  }
+  __device__ __forceinline__ Work(const TcParams &p, uint32_t n_mt)
+      : item(blockIdx.x), items(n_mt * (uint32_t)p.n_tiles * (uint32_t)p.slices), chunks((uint32_t)p.chunks), slices((uint32_t)p.slices) {}
   __device__ __forceinline__ bool next() {
-    if (pos >= end) return false;
-    tile = pos / chunks;
-    c0 = pos - tile * chunks;
-    c1 = split ? min(chunks, c0 + (end - pos)) : chunks;
-    pos += split ? c1 - c0 : gridDim.x * chunks;
+    if (item >= items) return false;
+    tile = item / slices;
+    slice = item - tile * slices;
+    c0 = slice * chunks / slices;
+    c1 = (slice + 1) * chunks / slices;
+    item += gridDim.x;
     return true;
   }
-  // chunks of this CTA, before the first next()
-  __device__ __forceinline__ uint32_t chunks_of_cta() const {
-    if (split) return end - pos;
-    const uint32_t tiles = total / chunks;
-    return blockIdx.x < tiles ? (tiles - blockIdx.x + gridDim.x - 1) / gridDim.x * chunks : 0u;
+  __device__ __forceinline__ bool last() const { return item >= items; }     // of the item that next() has set
+};
+
+// The accumulators of consecutive tiles.  Two sets take turns, so that a tile is summed while the one before it is drained;
+// a tile of two accumulators that are wider than half a set (`wide`) takes both sets.
+template <int NMAX>
+struct Accumulators {
+  static constexpr uint32_t kCount = NMAX <= 32 ? 4 : 2, kSetCols = kCount / 2 * NMAX;
+  uint32_t turn = 0, used[2] = {0, 0};
+  uint32_t set, use;              // of the current tile; use: how often the set was used before
+  uint32_t col, second;           // first column, distance of the second accumulator
+  bool wide;
+  __device__ __forceinline__ void next(bool two, int rows) {
+    wide = two && (kCount == 2 && rows > NMAX / 2);
+    set = wide ? 0u : turn;
+    turn = wide ? 0u : turn ^ 1;
+    use = set ? used[1]++ : used[0]++;
+    col = set * kSetCols;
+    second = !two ? 0u : kCount == 4 || wide ? (uint32_t)NMAX : (uint32_t)NMAX / 2;
   }
-  __device__ __forceinline__ bool last() const { return pos >= end; }     // of the segment that next() has set
-  __device__ __forceinline__ bool whole() const { return c1 - c0 == chunks; }
 };
 
 template <int NMAX, int KS, int TEAMS, int SLOTS, int XK, int XSTAGES, int PSTAGES>
@@ -168,10 +172,8 @@ struct SmemLayout {
   static constexpr int kXRing = XSTAGES * kXBytes;
   static constexpr int kPackedBytes = PSTAGES * kChunkBytes;
   static constexpr int kScaleBytes = PSTAGES * kScaleSlotBytes;
-  static constexpr int kEpiBytes = kEpiWarps * kEpiScratch * 4;
   static constexpr int kBarBytes = (2 * SLOTS + 2 * XSTAGES + 2 * PSTAGES + 5) * 8 + 8;
-  static_assert(TEAMS * kTeamWarps * kEpiScratch * 4 <= kXRing, "scratch of the conversion warps");
-  static constexpr int kTotal = kXRing + kPackedBytes + kScaleBytes + kEpiBytes + kBarBytes + 1024;
+  static constexpr int kTotal = kXRing + kPackedBytes + kScaleBytes + kBarBytes + 1024;
 };
 
 __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
@@ -272,26 +274,35 @@ __device__ __forceinline__ void convert32(const uint4 &packed, const DqParam &d,
   }
 }
 
-// One unary post-op on a thread's 16 values; the switch is outside the element loop so that its code exists once.
-__device__ __forceinline__ void unary_post16(float (&v)[4][4], int id) {
+// One unary post-op on a thread's 16 values; the switch is outside the element loop so that its code exists once.  The two
+// short ones are unrolled; the others go through four values at a time, because fetching a long straight run of code
+// that is executed once takes longer than the loop.
+__device__ __forceinline__ void unary_post16(float (&v)[16], int id) {
+  if (id == ZT_POST_RELU) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) v[j] = unary_post(v[j], ZT_POST_RELU);
+    return;
+  }
+  if (id == ZT_POST_SILU) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) v[j] = unary_post(v[j], ZT_POST_SILU);
+    return;
+  }
 #pragma unroll 1
   for (int q = 0; q < 4; ++q) {
+    // the first four, then rotate: after four rounds every value is back in its place
     float w[4];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) w[e] = q == 0 ? v[0][e] : q == 1 ? v[1][e] : q == 2 ? v[2][e] : v[3][e];
+    for (int e = 0; e < 4; ++e) w[e] = unary_post(v[e], id);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) w[e] = unary_post(w[e], id);
+    for (int e = 0; e < 12; ++e) v[e] = v[e + 4];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      if (q == 0) v[0][e] = w[e];
-      if (q == 1) v[1][e] = w[e];
-      if (q == 2) v[2][e] = w[e];
-      if (q == 3) v[3][e] = w[e];
-    }
+    for (int e = 0; e < 4; ++e) v[12 + e] = w[e];
   }
 }
 
-// The MMAs of one stage, 16 k each: A at consecutive columns of tensor memory, B by descriptor; then the commits that
+// The MMAs of one stage, 16 k each: A at consecutive columns of tensor memory, B by descriptor, the second 64 k into the
+// accumulator `d2`; then the commits that
 // free the converted slot and, when `free_x`, the activation slot.  Issued by the lane whose `leader` is set.  A completed
 // barrier wait takes its thread about 200 cycles, a third of a stage, so the barriers of the next stage are
 // tested in the same straight line of code: their answer arrives while the MMAs are being issued.
@@ -299,8 +310,8 @@ template <int N>
 struct MmaStage;
 template <>
 struct MmaStage<4> {
-  static __device__ __forceinline__ void issue(uint32_t leader, uint32_t d, uint32_t a, const uint64_t (&b)[4], uint32_t idesc,
-                                               uint32_t accumulate, uint32_t bar_a, uint32_t bar_x, uint32_t free_x,
+  static __device__ __forceinline__ void issue(uint32_t leader, uint32_t d, uint32_t, uint32_t a, const uint64_t (&b)[4],
+                                               uint32_t idesc, uint32_t accumulate, uint32_t, uint32_t bar_a, uint32_t bar_x, uint32_t free_x,
                                                uint32_t next_a, uint32_t par_a, uint32_t next_x, uint32_t par_x,
                                                uint32_t &ready) {
     asm volatile(
@@ -324,30 +335,32 @@ struct MmaStage<4> {
 };
 template <>
 struct MmaStage<8> {
-  static __device__ __forceinline__ void issue(uint32_t leader, uint32_t d, uint32_t a, const uint64_t (&b)[8], uint32_t idesc,
-                                               uint32_t accumulate, uint32_t bar_a, uint32_t bar_x, uint32_t free_x,
+  static __device__ __forceinline__ void issue(uint32_t leader, uint32_t d, uint32_t d2, uint32_t a, const uint64_t (&b)[8],
+                                               uint32_t idesc, uint32_t accumulate, uint32_t accumulate2, uint32_t bar_a, uint32_t bar_x, uint32_t free_x,
                                                uint32_t next_a, uint32_t par_a, uint32_t next_x, uint32_t par_x,
                                                uint32_t &ready) {
     asm volatile(
-        "{\n\t.reg .pred pa, px, pl, pc, pt;\n\t"
+        "{\n\t.reg .pred pa, px, pl, pc, pt, pd;\n\t"
         "mbarrier.test_wait.parity.shared::cta.b64 pa, [%9], %10;\n\t"
         "mbarrier.test_wait.parity.shared::cta.b64 px, [%11], %12;\n\t"
         "setp.ne.b32 pl, %1, 0;\n\tsetp.ne.b32 pc, %5, 0;\n\tsetp.eq.b32 pt, 0, 0;\n\t"
+        "setp.ne.b32 pd, %22, 0;\n\t"
         "{.reg .b32 t; add.u32 t, %3, 0; @pl tcgen05.mma.cta_group::1.kind::f16 [%2], [t], %13, %4, pc;}\n\t"
         "{.reg .b32 t; add.u32 t, %3, 8; @pl tcgen05.mma.cta_group::1.kind::f16 [%2], [t], %14, %4, pt;}\n\t"
         "{.reg .b32 t; add.u32 t, %3, 16; @pl tcgen05.mma.cta_group::1.kind::f16 [%2], [t], %15, %4, pt;}\n\t"
         "{.reg .b32 t; add.u32 t, %3, 24; @pl tcgen05.mma.cta_group::1.kind::f16 [%2], [t], %16, %4, pt;}\n\t"
-        "{.reg .b32 t; add.u32 t, %3, 32; @pl tcgen05.mma.cta_group::1.kind::f16 [%2], [t], %17, %4, pt;}\n\t"
-        "{.reg .b32 t; add.u32 t, %3, 40; @pl tcgen05.mma.cta_group::1.kind::f16 [%2], [t], %18, %4, pt;}\n\t"
-        "{.reg .b32 t; add.u32 t, %3, 48; @pl tcgen05.mma.cta_group::1.kind::f16 [%2], [t], %19, %4, pt;}\n\t"
-        "{.reg .b32 t; add.u32 t, %3, 56; @pl tcgen05.mma.cta_group::1.kind::f16 [%2], [t], %20, %4, pt;}\n\t"
+        "{.reg .b32 t; add.u32 t, %3, 32; @pl tcgen05.mma.cta_group::1.kind::f16 [%21], [t], %17, %4, pd;}\n\t"
+        "{.reg .b32 t; add.u32 t, %3, 40; @pl tcgen05.mma.cta_group::1.kind::f16 [%21], [t], %18, %4, pt;}\n\t"
+        "{.reg .b32 t; add.u32 t, %3, 48; @pl tcgen05.mma.cta_group::1.kind::f16 [%21], [t], %19, %4, pt;}\n\t"
+        "{.reg .b32 t; add.u32 t, %3, 56; @pl tcgen05.mma.cta_group::1.kind::f16 [%21], [t], %20, %4, pt;}\n\t"
         "@pl tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%6];\n\t"
         "setp.ne.and.b32 pl, %8, 0, pl;\n\t"
         "@pl tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%7];\n\t"
         "and.pred pa, pa, px;\n\tselp.u32 %0, 1, 0, pa;\n\t}"
         : "=r"(ready)
         : "r"(leader), "r"(d), "r"(a), "r"(idesc), "r"(accumulate), "r"(bar_a), "r"(bar_x), "r"(free_x), "r"(next_a),
-          "r"(par_a), "r"(next_x), "r"(par_x), "l"(b[0]), "l"(b[1]), "l"(b[2]), "l"(b[3]), "l"(b[4]), "l"(b[5]), "l"(b[6]), "l"(b[7])
+          "r"(par_a), "r"(next_x), "r"(par_x), "l"(b[0]), "l"(b[1]), "l"(b[2]), "l"(b[3]), "l"(b[4]), "l"(b[5]), "l"(b[6]), "l"(b[7]),
+          "r"(d2), "r"(accumulate2)
         : "memory");
   }
 };
@@ -369,14 +382,14 @@ __global__ void __launch_bounds__(threads_for(TEAMS), 1) woq_tcgen05_kernel(cons
   static_assert(TEAMS % kSPC == 0, "a team takes the same stage of every chunk that it visits");
   constexpr int kTeamsPerChunk = kSPC;
   constexpr uint32_t kACols = KS / 2;                    // tensor-memory columns of a converted stage
-  constexpr uint32_t kABase = 2 * NMAX;                  // after the two accumulators
+  constexpr bool kTwoAccs = KS == 128;                   // may sum a tile in two accumulators, a stage's halves in one each
+  constexpr uint32_t kABase = Accumulators<NMAX>::kCount * NMAX;   // the converted stages follow the accumulators
   static_assert(kABase + SLOTS * kACols <= 512, "tensor memory");
   extern __shared__ unsigned char smem_dyn[];
   unsigned char *smem = smem_dyn + ((1024u - (smem_u32(smem_dyn) & 1023u)) & 1023u);
   unsigned char *packed = smem + L::kXRing;
   unsigned char *sc_ring = packed + L::kPackedBytes;
-  float *epi_scratch = reinterpret_cast<float *>(sc_ring + L::kScaleBytes);
-  uint64_t *full_a = reinterpret_cast<uint64_t *>(sc_ring + L::kScaleBytes + L::kEpiBytes);   // converted
+  uint64_t *full_a = reinterpret_cast<uint64_t *>(sc_ring + L::kScaleBytes);   // converted
   uint64_t *empty_a = full_a + SLOTS;        // multiplied
   uint64_t *full_x = empty_a + SLOTS;        // activations landed
   uint64_t *empty_x = full_x + XSTAGES;      // multiplied
@@ -384,7 +397,7 @@ __global__ void __launch_bounds__(threads_for(TEAMS), 1) woq_tcgen05_kernel(cons
   uint64_t *empty_p = full_p + PSTAGES;      // packed chunk read by its teams
   uint64_t *tmem_full = empty_p + PSTAGES;   // [2]
   uint64_t *tmem_empty = tmem_full + 2;      // [2]
-  uint64_t *last_full = tmem_empty + 2;      // accumulator of the CTA's last segment
+  uint64_t *last_full = tmem_empty + 2;      // accumulator of the CTA's last item
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(last_full + 1);
 
   const int warp = tc::uniform_warp(), lane = threadIdx.x & 31;
@@ -428,9 +441,10 @@ __global__ void __launch_bounds__(threads_for(TEAMS), 1) woq_tcgen05_kernel(cons
   const uint32_t tmem_base = *tmem_slot;
   grid_launch_dependents();
 
-  // Every role walks the same segments, chunks and stages.  A stage past the end of K is void: nothing is loaded,
+  // Every role walks the same items, chunks and stages.  A stage past the end of K is void: nothing is loaded,
   // converted or multiplied, its barriers complete all the same, so ring positions stay aligned with chunks.
   Work wk(p, n_mt);
+  const bool two = kTwoAccs && p.accs == 2;
   // the producers and the issuer run as whole warps, lane 0 issuing
   const bool leader = tc::elect_one();
 
@@ -509,17 +523,18 @@ __global__ void __launch_bounds__(threads_for(TEAMS), 1) woq_tcgen05_kernel(cons
       const uint32_t x_field0 = (uint32_t)d0 | ((smem_u32(smem) & 0x3FFFF) >> 4);
       const uint32_t full_a0 = smem_u32(full_a), empty_a0 = smem_u32(empty_a);
       const uint32_t full_x0 = smem_u32(full_x), empty_x0 = smem_u32(empty_x);
-      uint32_t s = 0, ph = 0, xs = 0, xph = 0, local = 0;
+      uint32_t s = 0, ph = 0, xs = 0, xph = 0;
+      Accumulators<NMAX> acc;
       uint32_t ready = 0;
       while (wk.next()) {
         const TileInfo t = decode_tile(p, wk.tile, n_mt);
-        const uint32_t buf = local & 1, use = local >> 1;
-        ++local;
+        acc.next(two, t.rows);
         const uint32_t idesc = tc::instr_desc(1u, 1u, 1u, kBN, (uint32_t)((t.rows + 15) & ~15));
-        ok = ok && tc::warp_wait(smem_u32(&tmem_empty[buf]), (use & 1) ^ 1);
+        ok = ok && tc::warp_wait(smem_u32(&tmem_empty[acc.set]), (acc.use & 1) ^ 1);
+        if (acc.wide) ok = ok && tc::warp_wait(smem_u32(&tmem_empty[1]), (acc.used[1] & 1) ^ 1);
         if (!ok) tc::report_timeout(p.status, kStatusMmaTimeout);
         tc::fence_after_sync();
-        const uint32_t d_tmem = tmem_base + buf * NMAX;
+        const uint32_t d_tmem = tmem_base + acc.col, d_tmem2 = d_tmem + acc.second;
         uint32_t accumulate = 0;
         int k = (int)wk.c0 * kChunkK;
         const uint32_t stages = (wk.c1 - wk.c0) * kSPC;
@@ -550,9 +565,9 @@ __global__ void __launch_bounds__(threads_for(TEAMS), 1) woq_tcgen05_kernel(cons
             uint64_t b[KS / 16];
 #pragma unroll
             for (int j = 0; j < KS / 16; ++j) b[j] = tc::smem_desc_from_words(b_lo + (j >> 2) * block + 2 * (j & 3), desc_hi);
-            MmaStage<KS / 16>::issue(leader, d_tmem, a, b, idesc, accumulate, bar_a, bar_x, free_x, full_a0 + s * 8, ph,
-                                     full_x0 + xs * 8, xph, ready);
-          } else {
+            MmaStage<KS / 16>::issue(leader, d_tmem, d_tmem2, a, b, idesc, accumulate, two ? accumulate : 1u, bar_a, bar_x, free_x,
+                                     full_a0 + s * 8, ph, full_x0 + xs * 8, xph, ready);
+          } else {                            // the end of K: the first 64 k of the stage at most
             if (leader) {
               for (int j = 0; j < steps; ++j)
                 tc::mma_f16_ts(d_tmem, a + 8 * j, tc::smem_desc_from_words(b_lo + (j >> 2) * block + 2 * (j & 3), desc_hi), idesc,
@@ -566,7 +581,7 @@ __global__ void __launch_bounds__(threads_for(TEAMS), 1) woq_tcgen05_kernel(cons
           ready = __all_sync(0xffffffffu, ready);
           accumulate = 1;
         }
-        if (leader) tc::mma_commit(wk.last() ? last_full : &tmem_full[buf]);
+        if (leader) tc::mma_commit(wk.last() ? last_full : &tmem_full[acc.set]);
         __syncwarp();
       }
     }
@@ -585,13 +600,16 @@ __global__ void __launch_bounds__(threads_for(TEAMS), 1) woq_tcgen05_kernel(cons
     constexpr uint32_t kStep = TEAMS / kSPC;
     const uint32_t j = team % kSPC;
     const uint32_t row0 = smem_u32(packed) + row * 128 + (((j * kSub) ^ row_x) << 4);   // piece u: ^ (u << 4)
-    // Chunks of this CTA in ring order, and where the next of this team's stages lies in its tile
-    uint32_t left = wk.chunks_of_cta();
-    const uint32_t skip = team / kSPC;
-    uint32_t c = wk.pos - wk.pos / wk.chunks * wk.chunks + skip;
-    while (c >= wk.chunks) c -= wk.chunks;
-    left = left > skip ? (left - skip + kStep - 1) / kStep : 0;              // visits of this team
-    uint32_t ps = skip % PSTAGES, pph = 0;               // packed ring: slot, parity
+    uint32_t c = team / kSPC, end = 0;                   // this team's next chunk, end of the item it is counted in
+    auto next_chunk = [&]() {
+      while (c >= end) {
+        if (!wk.next()) return false;
+        c += wk.c0 - end;
+        end = wk.c1;
+      }
+      return true;
+    };
+    uint32_t ps = c % PSTAGES, pph = 0;                  // packed ring: slot, parity
     uint32_t e_ph = 1;                                   // parity of the slot's "free" barrier
     bool ok = true;
 
@@ -626,8 +644,6 @@ __global__ void __launch_bounds__(threads_for(TEAMS), 1) woq_tcgen05_kernel(cons
       }
     };
     auto next_stage = [&]() {
-      c += kStep;
-      while (c >= wk.chunks) c -= wk.chunks;
       ps += kStep;
       if (ps >= PSTAGES) {
         ps -= PSTAGES;
@@ -637,7 +653,7 @@ __global__ void __launch_bounds__(threads_for(TEAMS), 1) woq_tcgen05_kernel(cons
     if (p.staged_gpc) {
       // groups are at least 128 k wide: one scale per stage, in the chunk's slot
       const uint32_t sc_off = ((p.staged_gpc == 2 ? (j * KS) >> 7 : 0u) * kBN + row) * (kScaleDtype == ZT_F32 ? 4 : 2);
-      for (; left > 0; --left) {
+      for (; next_chunk(); c += kStep) {
         ok = ok && tc::warp_wait(smem_u32(&full_p[ps]), pph);
         const unsigned char *slot = sc_ring + ps * kScaleSlotBytes + sc_off;
         const DqParam d = dq_param<MODE>(load_as_float(slot, 0, kScaleDtype),
@@ -650,7 +666,7 @@ __global__ void __launch_bounds__(threads_for(TEAMS), 1) woq_tcgen05_kernel(cons
       // of this team's stages ahead
       Work fw(p, n_mt);
       int64_t f_base = 0;
-      uint32_t f_i = 0, f_n = 0, f_it = 0;               // stage within the segment, stages of it, ring position
+      uint32_t f_i = 0, f_n = 0, f_it = 0;               // stage within the item, stages of it, ring position
       float ns[kSub], nz[kSub];
       auto fetch = [&]() {
         for (;;) {
@@ -691,7 +707,7 @@ __global__ void __launch_bounds__(threads_for(TEAMS), 1) woq_tcgen05_kernel(cons
         ++f_it;
       };
       fetch();
-      for (; left > 0; --left) {
+      for (; next_chunk(); c += kStep) {
         DqParam d[kSub];
 #pragma unroll
         for (int u = 0; u < kSub; ++u) d[u] = dq_param<MODE>(ns[u], kAsym ? nz[u] : 0.f);
@@ -708,140 +724,86 @@ __global__ void __launch_bounds__(threads_for(TEAMS), 1) woq_tcgen05_kernel(cons
     }
     if (!ok && lane == 0) tc::report_timeout(p.status, kStatusConvertTimeout);
   }
-  // ---------------- epilogue: the epilogue warps; for a CTA's last segment the conversion warps too ----------------
-  // A job is 16 tokens x 32 columns of the accumulator.  The last segment is the part of a launch that nothing
+  // ---------------- epilogue: the epilogue warps; for a CTA's last item the conversion warps too ----------------
+  // A job is 16 tokens x 32 columns of the accumulator; a lane holds one column, so that loads and stores of a token's
+  // outputs are 64 contiguous bytes (as wide as a transposition through shared memory makes them, which cost 20 more
+  // shared-memory accesses and two barriers per job).  The last item is the part of a launch that nothing
   // overlaps, and by then the conversion teams are idle: with them a 128-token tile is drained by twenty warps
-  // instead of four (their scratch lies in the activation ring, which the last MMAs have read).
+  // instead of four.
   grid_dependency_wait();                // output, partial sums and post-op operands are shared with earlier work
   const bool epi_warp = warp < kFirstTeam;
   const uint32_t group = epi_warp ? 0u : 1u + (uint32_t)(warp - kFirstTeam) / kTeamWarps;
   const int quarter = warp & 3;          // tensor-memory lanes 32*quarter .. +31
-  float *scratch = epi_warp ? epi_scratch + (warp - 3) * kEpiScratch
-                            : reinterpret_cast<float *>(smem) + (warp - kFirstTeam) * kEpiScratch;
-  const int sub_row = lane >> 3, col4 = (lane & 7) * 4;   // a lane's token row within a group of 4, its four columns
-  // 8-byte accesses: rows of y start on 8-byte boundaries, and so do those of the binary post-op operands
-  const bool vec = (p.N & 3) == 0 && (reinterpret_cast<uintptr_t>(p.y) & 7) == 0;
-  bool vec_post = vec;
-#pragma unroll
-  for (int o = 0; o < ZT_MAX_POST_OPS; ++o) vec_post = vec_post && (reinterpret_cast<uintptr_t>(p.post.bufs[o]) & 7) == 0;
-  uint32_t local = 0;
+  Accumulators<NMAX> acc;
   bool ok = true;
   Work wd(p, n_mt);
   while (wd.next()) {
     const bool last = wd.last();
-    const uint32_t buf = local & 1, use = local >> 1;
-    ++local;
-    if (!last && !epi_warp) continue;
     const TileInfo ti = decode_tile(p, wd.tile, n_mt);
-    const int nq = ti.n0 + quarter * 32 + col4;           // first of this lane's output columns
-    float bias4[4] = {0.f, 0.f, 0.f, 0.f};
-    if (p.bias) {
+    acc.next(two, ti.rows);
+    if (!last && !epi_warp) continue;
+    const int n = ti.n0 + quarter * 32 + lane;            // this lane's output column
+    const bool live = n < p.N;
+    const float bias = p.bias && !p.partial && live ? load_as_float(p.bias, n, p.bias_dtype) : 0.f;
+    // operands of the first two binary post-ops for a job (two tokens' bf16 to a register), fetched before its sums are awaited
+    uint32_t operand[2][8];
+    auto request = [&](int job) {
+      const int rows = live ? min(16, ti.rows - job * 16) : 0;
 #pragma unroll
-      for (int e = 0; e < 4; ++e)
-        if (nq + e < p.N) bias4[e] = load_as_float(p.bias, nq + e, p.bias_dtype);
-    }
-    // A tile that spans CTAs cta_first .. cta_last: a CTA's piece goes to its slot 0 when its range starts in this
-    // tile, else to its slot 1; only the first CTA's range can start before the tile.
-    const bool whole = wd.whole();
-    uint32_t cta_first = 0, cta_last = 0, first_slot = 0;
-    if (!whole) {
-      cta_first = wd.cta_of(wd.tile * wd.chunks);
-      cta_last = wd.cta_of(wd.tile * wd.chunks + wd.chunks - 1);
-      first_slot = wd.first_of(cta_first) < wd.tile * wd.chunks ? 1u : 0u;
-    }
-    ok = ok && tc::warp_wait_idle(last ? smem_u32(last_full) : smem_u32(&tmem_full[buf]), last ? 0u : (use & 1));
+      for (int o = 0; o < 2; ++o) {
+        const uint16_t *src = reinterpret_cast<const uint16_t *>(p.post.bufs[o]);
+        if (!src) continue;
+        src += (int64_t)(ti.m0 + job * 16) * p.N + n;
+#pragma unroll
+        for (int j = 0; j < 16; j += 2, src += 2 * (int64_t)p.N)
+          operand[o][j / 2] = (j < rows ? (uint32_t)src[0] : 0u) | (j + 1 < rows ? (uint32_t)src[p.N] << 16 : 0u);
+      }
+    };
+    const bool with_operands = p.post.bufs[0] != nullptr && !p.partial;
+    const int jobs = (ti.rows + 15) >> 4, stride = last ? TEAMS + 1 : 1, job0 = last ? (int)group : 0;
+    if (with_operands && job0 < jobs) request(job0);
+    ok = ok && tc::warp_wait_idle(last ? smem_u32(last_full) : smem_u32(&tmem_full[acc.set]), last ? 0u : (acc.use & 1));
     if (!ok && lane == 0) tc::report_timeout(p.status, kStatusEpilogueTimeout);
     tc::fence_after_sync();
-    const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + buf * NMAX;
-    const uint32_t jobs = (uint32_t)(ti.rows + 15) >> 4;
-    const uint32_t job0 = last ? group : 0u, stride = last ? (uint32_t)TEAMS + 1u : 1u;
-    const uint32_t mine = jobs > job0 ? (jobs - job0 + stride - 1) / stride : 0u;     // jobs of this warp
-    // 16 tokens of the accumulator, transposed through scratch: v[q][e] = token r0 + 4 q, column nq + e
-    auto drain = [&](uint32_t job, float (&v)[4][4]) {
-      uint32_t r[16];
-      tc::tmem_ld_32x32b_x16(t_row + job * 16, r);
-      tc::tmem_ld_wait();
-#pragma unroll
-      for (int j = 0; j < 16; ++j) scratch[j * kEpiRowStride + lane] = __uint_as_float(r[j]);
-      __syncwarp();
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const float4 t4 = *reinterpret_cast<const float4 *>(&scratch[(q * 4 + sub_row) * kEpiRowStride + col4]);
-        v[q][0] = t4.x;
-        v[q][1] = t4.y;
-        v[q][2] = t4.z;
-        v[q][3] = t4.w;
-      }
-      __syncwarp();                                      // scratch is rewritten by the next job
-    };
-    auto piece_of = [&](uint32_t cta, uint32_t job) {
-      const uint32_t slot = 2 * cta + (cta == cta_first ? first_slot : 0u);
-      return reinterpret_cast<float4 *>(p.partial) + (size_t)((slot * 4 + quarter) * (NMAX / 16) + job) * 128 + lane;
-    };
-    uint32_t todo = (1u << mine) - 1u;                   // jobs to finish, by position in this warp's list
-    if (!whole) {
+    const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc.col;
+    // the second accumulator, unless the item has only 64 k (a tail of K)
+    const bool add_second = two && min(p.K, (int)wd.c1 * kChunkK) - (int)wd.c0 * kChunkK > 64;
 #pragma unroll 1
-      for (uint32_t i = 0; i < mine; ++i) {
-        float v[4][4];
-        drain(job0 + i * stride, v);
-        float4 *dst = piece_of(blockIdx.x, job0 + i * stride);
+    for (int job = job0; job < jobs; job += stride) {
+      // rows past the valid ones belong to nobody, or to the next expert
+      const int rows = live ? min(16, ti.rows - job * 16) : 0;
+      const int64_t row0 = ti.m0 + job * 16, at = row0 * p.N + n;
+      float v[16];
+      {
+        uint32_t r[16];
+        tc::tmem_ld_32x32b_x16(t_row + job * 16, r);
+        if (add_second) {
+          uint32_t r2[16];
+          tc::tmem_ld_32x32b_x16(t_row + acc.second + job * 16, r2);
+          tc::tmem_ld_wait();
 #pragma unroll
-        for (int q = 0; q < 4; ++q) __stcg(dst + q * 32, make_float4(v[q][0], v[q][1], v[q][2], v[q][3]));
-      }
-      // one fence for all of them (it takes about a microsecond), then a ticket each, a lane per job
-      __threadfence();
-      __syncwarp();
-      bool complete = false;
-      if (lane < (int)mine) {
-        unsigned int *ticket = p.tickets + (wd.tile * (NMAX / 16) + job0 + lane * stride) * 4 + quarter;
-        complete = atomicAdd(ticket, 1u) == cta_last - cta_first;
-        if (complete) *ticket = 0;                       // ready for the next launch
-      }
-      todo = __ballot_sync(0xffffffffu, complete);
-      __threadfence();
-    }
-#pragma unroll 1
-    for (; todo; todo &= todo - 1) {
-      const uint32_t job = job0 + (uint32_t)(__ffs(todo) - 1) * stride;
-      const int r0 = (int)job * 16 + sub_row;            // this lane's tokens of the tile: r0 + 4 q
-      const int64_t base0 = (int64_t)(ti.m0 + r0) * p.N + nq, step = (int64_t)4 * p.N;
-      // of the lane's four tokens, those that exist (rows past the valid ones belong to nobody, or to the next expert)
-      const int live = nq < p.N ? (ti.rows - r0 + 3) >> 2 : 0;
-      uint2 operand[2][4];                               // of the first two binary post-ops, requested early
-      if (vec_post) {
+          for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]) + __uint_as_float(r2[j]);
+        } else {
+          tc::tmem_ld_wait();
 #pragma unroll
-        for (int o = 0; o < 2; ++o)
-          if (p.post.bufs[o])
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-              if (q < live)
-                operand[o][q] = *reinterpret_cast<const uint2 *>(reinterpret_cast<const __nv_bfloat16 *>(p.post.bufs[o]) + base0 + q * step);
-      }
-      float v[4][4];
-      if (whole) {
-        drain(job, v);
-      } else {
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) v[q][e] = 0.f;
-#pragma unroll 4
-        for (uint32_t cta = cta_first; cta <= cta_last; ++cta) {   // in CTA order, whoever adds
-          const float4 *src = piece_of(cta, job);
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const float4 t4 = __ldcg(src + q * 32);
-            v[q][0] += t4.x;
-            v[q][1] += t4.y;
-            v[q][2] += t4.z;
-            v[q][3] += t4.w;
-          }
+          for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
         }
       }
+      if (!last && job + stride >= jobs) {               // read: the next tile may be summed here
+        tc::fence_before_sync();
+        __syncwarp();
+        tc::arrive_if(lane == 0, smem_u32(&tmem_empty[acc.set]));
+      }
+      if (p.partial) {                                   // the sums of this slice; bias and post-ops come when they are added
+        const int64_t pitch = (p.N + 3) & ~3;
+        float *dst = p.partial + ((int64_t)wd.slice * p.M + row0) * pitch + n;
 #pragma unroll
-      for (int q = 0; q < 4; ++q)
+        for (int j = 0; j < 16; ++j, dst += pitch)
+          if (j < rows) __stcg(dst, v[j]);
+        continue;
+      }
 #pragma unroll
-        for (int e = 0; e < 4; ++e) v[q][e] += bias4[e];
+      for (int j = 0; j < 16; ++j) v[j] += bias;
       int b = 0;
 #pragma unroll 1
       for (int o = 0; o < p.post.n_ops; ++o) {
@@ -850,43 +812,21 @@ __global__ void __launch_bounds__(threads_for(TEAMS), 1) woq_tcgen05_kernel(cons
           unary_post16(v, id);
           continue;
         }
-        const __nv_bfloat16 *other = reinterpret_cast<const __nv_bfloat16 *>(p.post.bufs[b]);
+        const uint16_t *src = b < 2 ? nullptr : reinterpret_cast<const uint16_t *>(p.post.bufs[b]) + at;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          float t[4];
-          if (vec_post) {
-            uint2 raw = b == 0 ? operand[0][q] : operand[1][q];
-            if (b >= 2 && q < live) raw = *reinterpret_cast<const uint2 *>(other + base0 + q * step);
-            t[0] = __uint_as_float(raw.x << 16);
-            t[1] = __uint_as_float(raw.x & 0xffff0000u);
-            t[2] = __uint_as_float(raw.y << 16);
-            t[3] = __uint_as_float(raw.y & 0xffff0000u);
-          } else {
-#pragma unroll
-            for (int e = 0; e < 4; ++e) t[e] = (q < live && nq + e < p.N) ? __bfloat162float(other[base0 + q * step + e]) : 0.f;
-          }
-#pragma unroll
-          for (int e = 0; e < 4; ++e) v[q][e] = id == ZT_POST_MUL ? v[q][e] * t[e] : v[q][e] + t[e];
+        for (int j = 0; j < 16; ++j) {
+          const uint32_t pair = b == 0 ? operand[0][j / 2] : operand[1][j / 2];
+          float t = __uint_as_float(j % 2 ? pair & 0xffff0000u : pair << 16);
+          if (src && j < rows) t = bf16_bits_to_float(src[(int64_t)j * p.N]);
+          v[j] = id == ZT_POST_MUL ? v[j] * t : v[j] + t;
         }
         ++b;
       }
+      __nv_bfloat16 *dst = p.y + at;
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        if (q >= live) continue;
-        __nv_bfloat16 *dst = p.y + base0 + q * step;
-        if (vec) {
-          *reinterpret_cast<uint2 *>(dst) = make_uint2(bf2_pack(v[q][0], v[q][1]), bf2_pack(v[q][2], v[q][3]));
-        } else {
-#pragma unroll
-          for (int e = 0; e < 4; ++e)
-            if (nq + e < p.N) dst[e] = __float2bfloat16_rn(v[q][e]);
-        }
-      }
-    }
-    if (!last) {
-      tc::fence_before_sync();
-      __syncwarp();
-      tc::arrive_if(lane == 0, smem_u32(&tmem_empty[buf]));
+      for (int j = 0; j < 16; ++j, dst += p.N)
+        if (j < rows) *dst = __float2bfloat16_rn(v[j]);
+      if (with_operands && job + stride < jobs) request(job + stride);
     }
   }
   }
@@ -896,6 +836,61 @@ __global__ void __launch_bounds__(threads_for(TEAMS), 1) woq_tcgen05_kernel(cons
   if (warp == 1) {
     tc::fence_after_sync();
     tc::tmem_dealloc(tmem_base, 512);
+  }
+}
+
+constexpr int kSliceThreads = 128;
+
+// y = post_ops(sum over the slices + bias), the slices in order, four columns per thread.  Bound by latency and, for many
+// rows, by L2: a launch of its own on the dependency of the one before it costs less than a meeting of the slices' CTAs at
+// the end of the main kernel (pieces to L2, fence, ticket, addition by the last to arrive: 5 - 10 us).
+__global__ void __launch_bounds__(kSliceThreads) woq_slices_kernel(const float *__restrict__ partial, int slices, int M, int N,
+                                                                   const void *__restrict__ bias, int bias_dtype,
+                                                                   const __grid_constant__ PostOpsDev post,
+                                                                   __nv_bfloat16 *__restrict__ y) {
+  grid_launch_dependents();
+  grid_dependency_wait();
+  const int quads_n = (N + 3) >> 2;
+  const int64_t quad = (int64_t)blockIdx.x * kSliceThreads + threadIdx.x;
+  if (quad >= (int64_t)M * quads_n) return;
+  const int64_t m = quad / quads_n;
+  const int n = (int)(quad - m * quads_n) * 4, live = min(4, N - n);
+  const int64_t base = m * N + n, step = (int64_t)M * quads_n * 4;
+  float v[4] = {0.f, 0.f, 0.f, 0.f};
+  const float *src = partial + quad * 4;
+#pragma unroll 4
+  for (int s = 0; s < slices; ++s) {
+    const float4 t = __ldcg(reinterpret_cast<const float4 *>(src + s * step));
+    v[0] += t.x;
+    v[1] += t.y;
+    v[2] += t.z;
+    v[3] += t.w;
+  }
+  int b = 0;
+#pragma unroll
+  for (int e = 0; e < 4; ++e)
+    if (bias && e < live) v[e] += load_as_float(bias, n + e, bias_dtype);
+#pragma unroll 1
+  for (int o = 0; o < post.n_ops; ++o) {
+    const int id = post.ids[o];
+    const bool binary = id == ZT_POST_MUL || id == ZT_POST_ADD;
+    const __nv_bfloat16 *other = binary ? reinterpret_cast<const __nv_bfloat16 *>(post.bufs[b++]) + base : nullptr;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      if (!binary) {
+        v[e] = unary_post(v[e], id);
+      } else if (e < live) {
+        const float t = __bfloat162float(other[e]);
+        v[e] = id == ZT_POST_MUL ? v[e] * t : v[e] + t;
+      }
+    }
+  }
+  if (live == 4 && (N & 3) == 0 && (reinterpret_cast<uintptr_t>(y) & 7) == 0) {
+    *reinterpret_cast<uint2 *>(y + base) = make_uint2(bf2_pack(v[0], v[1]), bf2_pack(v[2], v[3]));
+  } else {
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if (e < live) y[base + e] = __float2bfloat16_rn(v[e]);
   }
 }
 
@@ -986,9 +981,9 @@ int launch_cfg(const TcParams &p0, int scale_dtype, const void *x, int64_t x_row
       }
     }
   }
-  const int64_t tiles = (int64_t)(p.g_count ? max_row_tiles : p.m_tiles) * p.n_tiles;
+  const int64_t items = (int64_t)(p.g_count ? max_row_tiles : p.m_tiles) * p.n_tiles * p.slices;
   const int sms = sm_count();
-  const dim3 grid(p.split ? (unsigned)p.split : (unsigned)(tiles < sms ? tiles : sms));
+  const dim3 grid((unsigned)(items < sms ? items : sms));
   // every instantiation needs its own once-per-device attribute set-up
   static PerDeviceOnce configured[4];
   auto launch = [&](auto kern, int which) -> int {
@@ -1022,51 +1017,68 @@ int launch_any(int cap, const TcParams &p, int scale_dtype, const void *x, int64
 struct DensePlan {
   int cap;       // instantiation
   int m_tiles, bt;
-  int split;     // CTAs that share the chunks of all tiles; 0 = whole tiles
+  int slices;    // of K, per tile
+  int accs;      // accumulators per item
 };
 int cap_for(int64_t rows) { return rows <= 32 ? 32 : rows <= 64 ? 64 : rows <= 128 ? 128 : 192; }
+// How many sums a tile's K is at least divided among.  The tensor core's fp32 accumulation truncates, so its error grows
+// with the number of products added to one accumulator (relative to the result's root mean square 3.5e-6 for 4096 k in
+// one sum, 1.6e-6 in two; 8192 k: 7.7e-6 in one, 1.6e-6 in four).  Up to 128 rows two accumulators take alternate blocks of
+// 64 k, and up to 256 rows K is cut into as many equal slices of whole chunks as the SMs can work on at once.
+int64_t min_sums(int64_t M, int64_t N, int64_t K) {
+  if (M > 256) return 1;
+  const int64_t room = std::min<int64_t>(kMaxSlices, sm_count() / ceil_div<int64_t>(N, kBN)), chunks = K / kChunkK;
+  int64_t slices = 1;
+  for (int64_t ks = 2; ks <= room && K % kChunkK == 0; ++ks)
+    if (chunks % ks == 0) slices = ks;
+  return M <= 128 ? 2 * slices : slices;
+}
 
-// The number of row tiles, and whether the chunks of all tiles are shared out, by estimated cycles.  A 128 x 64 block
-// takes the slower of the conversion pipeline (about 300 cycles measured) and the MMAs (2 per token, and about 90
-// around them).  Sharing out costs about 20,000 cycles at the end of the launch (pieces to L2, fence, tickets, the
-// addition; 10,000 - 21,000 measured), so it pays for few tiles with a long K only: M = 32, 4096 -> 14336 takes 13.7 us
-// with whole tiles on 112 SMs and 16.6 shared by 148; M = 64, 4096 -> 4096 12.5 and 15.7.
-DensePlan dense_plan(int64_t M, int64_t N, int64_t K, int hint, bool may_split) {
-  const int sms = sm_count();
-  const int64_t n_tiles = ceil_div<int64_t>(N, kBN), chunks = ceil_div<int64_t>(K, kChunkK);
-  const int64_t limit = hint > 0 ? std::min(hint, 192) : 192;
-  const int64_t first = ceil_div<int64_t>(M, limit);
+// The number of row tiles and of K slices by estimated cycles.  A 128 x 64 block takes the slower of the conversion
+// (350 cycles, 560 where it calculates in fp32) and the MMAs (2 per token, and about 90 around them), and then waits for its
+// operands out of L2 the longer, the more rows a tile has and the more SMs pull; adding slices up takes a launch of its own
+// (5000 cycles) and their way through L2.  The constants are fitted to 108 shapes of 130 - 1024 rows timed with every plan:
+// the chosen one is 1 % above the fastest in the mean and 11 % at most.  M = 192, 14336 -> 4096: 53 us in one slice, 22.5 in
+// four; M = 384: 39 as 2 x 2, 53 as three row tiles of whole K; M = 256, 2816 -> 5003: 14.0 whole, 21.6 in two slices.
+DensePlan dense_plan(int64_t M, int64_t N, int64_t K, bool fp32_conversion, bool may_slice) {
+  const int64_t sms = sm_count(), n_tiles = ceil_div<int64_t>(N, kBN), chunks = ceil_div<int64_t>(K, kChunkK);
+  const int64_t sums = may_slice ? min_sums(M, N, K) : M <= 128 ? 2 : 1, first = ceil_div<int64_t>(M, 192);
   DensePlan best{};
   double best_cost = 1e300;
-  for (int64_t mt = first; mt <= first + first / 2 + (hint > 0 ? 0 : 1) && mt <= ceil_div<int64_t>(M, 16); ++mt) {
-    const int64_t bt = ceil_div<int64_t>(ceil_div(M, mt), 16) * 16, tiles_m = ceil_div(M, bt);
-    const int64_t tiles = tiles_m * n_tiles;
-    const double chunk = 4.0 * std::max(300.0, 2.0 * (double)bt + 90.0);
-    double cost = (double)ceil_div<int64_t>(tiles, sms) * chunks * chunk;
-    int split = 0;
-    if (may_split && tiles * (cap_for(bt) / 4) <= kTickets) {
-      // at least two chunks per CTA, at most sixteen CTAs per tile
-      const int64_t ctas = std::min<int64_t>({(int64_t)sms, tiles * 16, std::max<int64_t>(tiles * chunks / 2, 1)});
-      const double c = (double)(tiles * chunks) / ctas * chunk + 20000.0;
-      if (ctas > 1 && c < cost) {
-        cost = c;
-        split = (int)ctas;
+  for (int64_t mt = first; mt <= first + first / 2 + 1 && mt <= ceil_div<int64_t>(M, 16); ++mt) {
+    const int64_t bt = ceil_div<int64_t>(ceil_div(M, mt), 16) * 16, tiles_m = ceil_div(M, bt), tiles = tiles_m * n_tiles;
+    const int64_t accs_max = bt <= 128 ? 2 : 1;
+    const double block = std::max(fp32_conversion ? 560.0 : 350.0, 2.0 * (double)bt + 90.0);
+    const int64_t least = std::min(ceil_div(sums, accs_max), chunks);
+    const int64_t most = may_slice ? std::max(least, std::min<int64_t>({sms / tiles, kMaxSlices, chunks})) : 1;
+    for (int64_t ks = std::max<int64_t>(least, 1); ks <= most; ++ks) {
+      if (ks > least && ceil_div(chunks, ks) == ceil_div(chunks, ks - 1)) continue;     // no shorter than with fewer
+      const double wait = 0.4 * (double)(bt + 36) * (double)std::min(tiles * ks, sms) / (double)sms;
+      double cost = (double)(ceil_div<int64_t>(tiles * ks, sms) * ceil_div(chunks, ks)) * 4.0 * (block + wait);
+      if (ks > 1) cost += 5000.0 + (double)(ks * M * N) / 400.0;
+      if (cost < best_cost) {
+        best_cost = cost;
+        best = {cap_for(bt), (int)tiles_m, (int)bt, (int)ks, ks < sums && accs_max == 2 ? 2 : 1};
       }
-    }
-    if (cost < best_cost) {
-      best_cost = cost;
-      best = {cap_for(bt), (int)tiles_m, (int)bt, split};
     }
   }
   return best;
 }
-size_t split_bytes(const DensePlan &d) {
-  return d.split ? (size_t)d.split * 2 * kBN * d.cap * sizeof(float) : 0;
+size_t slices_bytes(const DensePlan &d, int64_t M, int64_t N) {
+  return d.slices > 1 ? (size_t)d.slices * M * ((N + 3) & ~3) * sizeof(float) : 0;
 }
 
 }  // namespace
 
-size_t woq_tcgen05_workspace_bytes(int64_t M, int64_t N, int64_t K) { return split_bytes(dense_plan(M, N, K, 0, true)); }
+size_t woq_tcgen05_workspace_bytes(int64_t M, int64_t N, int64_t K) {
+  return std::max(slices_bytes(dense_plan(M, N, K, false, true), M, N), slices_bytes(dense_plan(M, N, K, true, true), M, N));
+}
+
+void woq_tcgen05_plan(int64_t M, int64_t N, int64_t K, bool fp32_conversion, int32_t *plan) {
+  const DensePlan d = dense_plan(M, N, K, fp32_conversion, true);
+  const int values[5] = {d.cap, d.m_tiles, d.bt, d.slices, d.accs};
+  std::copy(values, values + 5, plan);
+}
 
 bool woq_tcgen05_supported(const zt_woq_linear_args_t &a) {
   if (a.M < 1 || a.N < 1 || a.K < 64 || a.K % 64 != 0) return false;
@@ -1094,18 +1106,32 @@ int woq_tcgen05_launch(const zt_woq_linear_args_t &a, cudaStream_t st) {
   const int hint = (a.algo >> 8) & 0xffff;
   ZT_REQUIRE(hint == 0 || hint == 32 || hint == 64 || hint == 128 || hint == 256, ZT_UNSUPPORTED,
              "zt_woq_linear: unsupported token-tile width %d for the tcgen05 kernel", hint);
-  const bool may_split = hint == 0 && !(a.algo & ZT_ALGO_SINGLE_ISSUER) && a.workspace != nullptr;
-  DensePlan d = dense_plan(a.M, a.N, a.K, hint, may_split);
-  if (d.split && a.workspace_bytes < ZT_WOQ_COUNTER_BYTES + split_bytes(d)) d = dense_plan(a.M, a.N, a.K, hint, false);
+  const bool one_acc = (a.algo & ZT_ALGO_ONE_ACCUMULATOR) != 0, fp32_conversion = a.zeros && a.scale_dtype == ZT_F32;
+  DensePlan d = dense_plan(a.M, a.N, a.K, fp32_conversion, hint == 0 && !one_acc && a.workspace != nullptr);
+  if (d.slices > 1 && a.workspace_bytes < ZT_WOQ_COUNTER_BYTES + slices_bytes(d, a.M, a.N))
+    d = dense_plan(a.M, a.N, a.K, fp32_conversion, false);
+  if (hint > 0) {                      // the instantiation that takes tiles of this width (the widest: 192)
+    d.cap = hint == 256 ? 192 : hint;
+    d.m_tiles = (int)ceil_div<int64_t>(a.M, d.cap);
+    d.bt = (int)ceil_div<int64_t>(ceil_div<int64_t>(a.M, d.m_tiles), 16) * 16;
+    d.m_tiles = (int)ceil_div<int64_t>(a.M, d.bt);
+    d.accs = d.cap <= 128 ? 2 : 1;
+  }
+  if (one_acc) d.accs = 1;
   p.m_tiles = d.m_tiles;
   p.n_tiles = (int)ceil_div<int64_t>(a.N, kBN);
   p.bt = d.bt;
   p.chunks = (int)ceil_div<int64_t>(a.K, kChunkK);
+  p.slices = d.slices;
+  p.accs = d.accs;
   p.x_box = p.x_box2 = d.m_tiles == 1 ? (int)ceil_div<int64_t>(a.M, 8) * 8 : d.bt;   // 128-byte swizzle: 8-row atoms
-  p.split = d.split;
-  p.tickets = reinterpret_cast<unsigned int *>(a.workspace);
-  p.partial = d.split ? reinterpret_cast<float *>(reinterpret_cast<char *>(a.workspace) + ZT_WOQ_COUNTER_BYTES) : nullptr;
-  return launch_any(d.cap, p, a.scale_dtype, a.x, a.M, a.N, 0, st);
+  p.partial = d.slices > 1 ? reinterpret_cast<float *>(reinterpret_cast<char *>(a.workspace) + ZT_WOQ_COUNTER_BYTES) : nullptr;
+  const int rc = launch_any(d.cap, p, a.scale_dtype, a.x, a.M, a.N, 0, st);
+  if (rc != ZT_SUCCESS || d.slices == 1) return rc;
+  const int64_t quads = a.M * ceil_div<int64_t>(a.N, 4);
+  ZT_CUDA_OK(launch_overlapped(woq_slices_kernel, dim3((unsigned)ceil_div<int64_t>(quads, kSliceThreads)), dim3(kSliceThreads), (size_t)0, st,
+                               (const float *)p.partial, d.slices, p.M, p.N, p.bias, p.bias_dtype, p.post, p.y));
+  return launch_status("woq_slices_kernel");
 }
 
 // Grouped form for mixture-of-experts: `x` holds `total_rows` rows sorted by expert; `tiles` / `tile_count`
@@ -1126,6 +1152,8 @@ int woq_tcgen05_grouped_launch(const void *x, int64_t total_rows, int64_t N, int
   p.n_tiles = (int)ceil_div<int64_t>(N, kBN);
   p.bt = row_tile;
   p.chunks = (int)ceil_div<int64_t>(K, kChunkK);
+  p.slices = 1;
+  p.accs = row_tile <= 128 ? 2 : 1;
   p.x_box = row_tile > 64 ? 64 : row_tile;
   p.x_box2 = row_tile;
   p.g_count = tile_count;

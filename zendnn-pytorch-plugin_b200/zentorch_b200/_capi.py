@@ -17,7 +17,8 @@ ZT_BF16, ZT_F32, ZT_U8, ZT_S8 = 0, 1, 2, 3
 ZT_MAX_POST_OPS = 4
 ZT_WOQ_COUNTER_BYTES = 16384
 ZT_ALGO_AUTO, ZT_ALGO_GENERIC, ZT_ALGO_SKINNY, ZT_ALGO_TCGEN05 = 0, 1, 2, 3
-ZT_ALGO_SINGLE_ISSUER = 1 << 24
+ZT_ALGO_ONE_ACCUMULATOR = 1 << 24
+ZT_ALGO_SINGLE_ISSUER = ZT_ALGO_ONE_ACCUMULATOR
 ZT_ACT_S8_SYM, ZT_ACT_U8_ASYM = 0, 1
 ZT_FLAG_WEIGHTS_VOLATILE = 1
 ZT_STATIC_SCRATCH_Q_BYTES, ZT_STATIC_SCRATCH_MAX_ROWS = 8 << 20, 16384
@@ -27,6 +28,7 @@ ZT_STATIC_SCRATCH_Q_BYTES, ZT_STATIC_SCRATCH_MAX_ROWS = 8 << 20, 16384
 # Every symbol include/zentorch_b200.h declares; the CPU test-suite checks the library exports all.
 EXPORTED_SYMBOLS = (
     "zt_last_error", "zt_version", "zt_device_supported", "zt_poll_device_status", "zt_selftest_expire_wait", "zt_debug_set_timeline",
+    "zt_debug_woq_plan",
     "zt_woq_linear_workspace_bytes", "zt_woq_linear", "zt_woq_repack_weight", "zt_woq_repack_from_int4pack",
     "zt_dynamic_qlinear_workspace_bytes", "zt_dynamic_qlinear", "zt_dynamic_quantize", "zt_int8_gemm_s32",
     "zt_int8_weight_rowsum", "zt_qlinear_prequantized", "zt_dynamic_qlinear_static",
@@ -116,6 +118,7 @@ def lib() -> C.CDLL:
     L.zt_poll_device_status.argtypes = [C.POINTER(C.c_int), C.c_int]
     L.zt_selftest_expire_wait.argtypes = [C.c_void_p]
     L.zt_debug_set_timeline.argtypes = [C.c_void_p, C.c_size_t]
+    L.zt_debug_woq_plan.argtypes = [C.c_int64, C.c_int64, C.c_int64, C.c_int32, C.POINTER(C.c_int32)]
     L.zt_woq_linear_workspace_bytes.restype = C.c_size_t
     L.zt_woq_linear_workspace_bytes.argtypes = [C.c_int64, C.c_int64, C.c_int64]
     L.zt_woq_linear.argtypes = [C.POINTER(WoqLinearArgs), C.c_void_p]
@@ -163,6 +166,13 @@ def poll_device_status(reset: bool = True) -> int:
         if torch_lib is not None:
             torch_lib.zentorch_b200_reset_workspaces()
     return st.value
+
+
+def woq_plan(m, n, k, fp32_conversion=False):
+    """zt_debug_woq_plan: (tile capacity, row tiles, rows per tile, K slices, accumulators) of the tensor-core kernel."""
+    plan = (C.c_int32 * 5)()
+    check(lib().zt_debug_woq_plan(m, n, k, 1 if fp32_conversion else 0, plan))
+    return tuple(plan)
 
 
 def _torch_boundary():
