@@ -244,11 +244,15 @@ __device__ __forceinline__ void convert32(const uint4 &packed, const DqParam &d,
   if (MODE == kAsymF32) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
+      const uint32_t w = words[i], high = w >> 20;
       float f[8];
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
-        const uint32_t bits = ((words[i] >> (4 * e)) & 0xFu) | 0x4B000000u;   // 2^23 + q
-        f[e] = fmaf(__uint_as_float(bits) - 8388616.0f, __uint_as_float(d.a), __uint_as_float(d.b));   // (q - 8) * s + z
+        // a nibble where it lies, as 2^23 + 16^j q; times 16^-j and without the offset it is q - 8, exactly
+        const int j = e < 5 ? e : e - 5;
+        const uint32_t bits = ((e < 5 ? w : high) & (0xFu << (4 * j))) | 0x4B000000u;
+        const float unit = 1.0f / (float)(1 << (4 * j));
+        f[e] = fmaf(fmaf(__uint_as_float(bits), unit, -8388608.0f * unit - 8.0f), __uint_as_float(d.a), __uint_as_float(d.b));
       }
 #pragma unroll
       for (int e = 0; e < 4; ++e) out[4 * i + e] = bf2_pack(f[2 * e], f[2 * e + 1]);
@@ -1035,7 +1039,7 @@ int64_t min_sums(int64_t M, int64_t N, int64_t K) {
 }
 
 // The number of row tiles and of K slices by estimated cycles.  A 128 x 64 block takes the slower of the conversion
-// (350 cycles, 560 where it calculates in fp32) and the MMAs (2 per token, and about 90 around them), and then waits for its
+// (350 cycles, 400 where it calculates in fp32) and the MMAs (2 per token, and about 90 around them), and then waits for its
 // operands out of L2 the longer, the more rows a tile has and the more SMs pull; adding slices up takes a launch of its own
 // (5000 cycles) and their way through L2.  The constants are fitted to 108 shapes of 130 - 1024 rows timed with every plan:
 // the chosen one is 1 % above the fastest in the mean and 11 % at most.  M = 192, 14336 -> 4096: 53 us in one slice, 22.5 in
@@ -1048,7 +1052,7 @@ DensePlan dense_plan(int64_t M, int64_t N, int64_t K, bool fp32_conversion, bool
   for (int64_t mt = first; mt <= first + first / 2 + 1 && mt <= ceil_div<int64_t>(M, 16); ++mt) {
     const int64_t bt = ceil_div<int64_t>(ceil_div(M, mt), 16) * 16, tiles_m = ceil_div(M, bt), tiles = tiles_m * n_tiles;
     const int64_t accs_max = bt <= 128 ? 2 : 1;
-    const double block = std::max(fp32_conversion ? 560.0 : 350.0, 2.0 * (double)bt + 90.0);
+    const double block = std::max(fp32_conversion ? 400.0 : 350.0, 2.0 * (double)bt + 90.0);
     const int64_t least = std::min(ceil_div(sums, accs_max), chunks);
     const int64_t most = may_slice ? std::max(least, std::min<int64_t>({sms / tiles, kMaxSlices, chunks})) : 1;
     for (int64_t ks = std::max<int64_t>(least, 1); ks <= most; ++ks) {
