@@ -76,9 +76,9 @@ constexpr int kPackedProducer = 2;
 constexpr int threads_for(int teams) { return 32 * (kFirstTeam + teams * kTeamWarps); }
 constexpr int kChunkK = 256;        // k per packed chunk: one 128-byte row of nibbles
 constexpr int kChunkBytes = kBN * 128;
-// per packed chunk: up to two groups x 128 columns of fp32 scales (1 KB), then the same for zero points
-constexpr int kScaleSlotBytes = 2048;
-constexpr int kZeroSlotOffset = 1024;
+// per packed chunk: up to eight groups x 128 columns of scales, then the same for zero points (8 KB when both are fp32; where
+// the activation ring leaves no room for that, tables that need more than 4 KB are read from global memory)
+__host__ __device__ constexpr int scale_slot_bytes(int nmax) { return nmax == 64 ? 4096 : 8192; }
 constexpr int kMaxSlices = 32;      // K slices of a tile
 
 // How a weight is dequantised (template parameter of the kernel).
@@ -103,7 +103,7 @@ struct TcParams {
   // grouped mode (g_count != nullptr)
   const int *g_count;         // number of row tiles
   const int4 *g_tiles;        // per row tile: {expert, first row, valid rows, 0}
-  // Scales (and zero points) staged in shared memory with every packed chunk: groups per chunk (1 or 2; 0 = the
+  // Scales (and zero points) staged in shared memory with every packed chunk: groups per chunk (1 .. 8; 0 = the
   // conversion threads fetch them from global memory), groups per expert.
   int staged_gpc, groups;
 };
@@ -171,7 +171,7 @@ struct SmemLayout {
   static constexpr int kXBytes = (XK / 64) * NMAX * 128;
   static constexpr int kXRing = XSTAGES * kXBytes;
   static constexpr int kPackedBytes = PSTAGES * kChunkBytes;
-  static constexpr int kScaleBytes = PSTAGES * kScaleSlotBytes;
+  static constexpr int kScaleBytes = PSTAGES * scale_slot_bytes(NMAX);
   static constexpr int kBarBytes = (2 * SLOTS + 2 * XSTAGES + 2 * PSTAGES + 5) * 8 + 8;
   static constexpr int kTotal = kXRing + kPackedBytes + kScaleBytes + kBarBytes + 1024;
 };
@@ -380,6 +380,7 @@ __global__ void __launch_bounds__(threads_for(TEAMS), 1) woq_tcgen05_kernel(cons
   constexpr bool kAsym = MODE == kAsymBf16 || MODE == kAsymF32;
   constexpr int kScaleDtype = (MODE == kSymF32 || MODE == kAsymF32) ? ZT_F32 : ZT_BF16;
   constexpr int kSPC = kChunkK / KS;                     // stages per chunk
+  constexpr uint32_t kScaleSlot = scale_slot_bytes(NMAX), kScaleSize = kScaleDtype == ZT_F32 ? 4 : 2;
   constexpr int kSPX = XK / KS;                           // stages per activation slot
   static_assert(XK % KS == 0 && kChunkK % XK == 0, "activation slots");
   static_assert(SLOTS % TEAMS == 0, "a slot belongs to one team");
@@ -457,7 +458,7 @@ __global__ void __launch_bounds__(threads_for(TEAMS), 1) woq_tcgen05_kernel(cons
     {
       const uint32_t full_p0 = smem_u32(full_p), empty_p0 = smem_u32(empty_p);
       const uint32_t packed0 = smem_u32(packed), sc0 = smem_u32(sc_ring);
-      const uint32_t chunk_tx = kChunkBytes + (kAsym ? 2u : 1u) * (uint32_t)p.staged_gpc * kBN * (kScaleDtype == ZT_F32 ? 4u : 2u);
+      const uint32_t chunk_tx = kChunkBytes + (kAsym ? 2u : 1u) * (uint32_t)p.staged_gpc * kBN * kScaleSize;
       uint32_t s = 0, ph = 1;
       bool ok = true;
       while (ok && wk.next()) {
@@ -474,8 +475,8 @@ __global__ void __launch_bounds__(threads_for(TEAMS), 1) woq_tcgen05_kernel(cons
           tc::expect_tx_if(leader, bar, chunk_tx);
           tc::load_2d_if(leader, packed0 + s * kChunkBytes, &tmap_w, bar, (int)c * (kChunkK / 8), row);
           if (p.staged_gpc) {
-            tc::load_2d_if(leader, sc0 + s * kScaleSlotBytes, &tmap_s, bar, t.n0, g0);
-            if (kAsym) tc::load_2d_if(leader, sc0 + s * kScaleSlotBytes + kZeroSlotOffset, &tmap_z, bar, t.n0, g0);
+            tc::load_2d_if(leader, sc0 + s * kScaleSlot, &tmap_s, bar, t.n0, g0);
+            if (kAsym) tc::load_2d_if(leader, sc0 + s * kScaleSlot + (uint32_t)p.staged_gpc * kBN * kScaleSize, &tmap_z, bar, t.n0, g0);
           }
           if (++s == PSTAGES) {
             s = 0;
@@ -655,19 +656,32 @@ __global__ void __launch_bounds__(threads_for(TEAMS), 1) woq_tcgen05_kernel(cons
       }
     };
     if (p.staged_gpc) {
-      // groups are at least 128 k wide: one scale per stage, in the chunk's slot
-      const uint32_t sc_off = ((p.staged_gpc == 2 ? (j * KS) >> 7 : 0u) * kBN + row) * (kScaleDtype == ZT_F32 ? 4 : 2);
+      // the group of a 32-k piece: its k within the chunk >> log2 of the group size (one group, if that is larger)
+      const uint32_t zero_off = (uint32_t)p.staged_gpc * kBN * kScaleSize, shift = p.staged_gpc == 1 ? 31u : (uint32_t)p.gs_log2;
       for (; next_chunk(); c += kStep) {
         ok = ok && tc::warp_wait(smem_u32(&full_p[ps]), pph);
-        const unsigned char *slot = sc_ring + ps * kScaleSlotBytes + sc_off;
-        const DqParam d = dq_param<MODE>(load_as_float(slot, 0, kScaleDtype),
-                                         kAsym ? load_as_float(slot + kZeroSlotOffset, 0, kScaleDtype) : 0.f);
-        convert_stage(ok ? min(kSub, (p.K - (int)(c * kChunkK + j * KS)) / 32) : 0, [&]() { return d; });
+        const unsigned char *slot = sc_ring + ps * kScaleSlot + row * kScaleSize;
+        uint32_t k = j * KS;
+        auto group_param = [&]() {
+          const unsigned char *at = slot + (k >> shift) * (kBN * kScaleSize);
+          return dq_param<MODE>(load_as_float(at, 0, kScaleDtype), kAsym ? load_as_float(at + zero_off, 0, kScaleDtype) : 0.f);
+        };
+        const int quads = ok ? min(kSub, (p.K - (int)(c * kChunkK + j * KS)) / 32) : 0;
+        if (p.gs_log2 >= 7) {                            // one group per stage
+          const DqParam d = group_param();
+          convert_stage(quads, [&]() { return d; });
+        } else {
+          convert_stage(quads, [&]() {
+            const DqParam d = group_param();
+            k += 32;
+            return d;
+          });
+        }
         next_stage();
       }
     } else {
-      // groups of 32 or 64 k, of no power of two, or tables that TMA cannot address: scales from global memory, one
-      // of this team's stages ahead
+      // groups of no power of two, or tables that TMA cannot address or that do not fit: scales from global memory, one of
+      // this team's stages ahead
       Work fw(p, n_mt);
       int64_t f_base = 0;
       uint32_t f_i = 0, f_n = 0, f_it = 0;               // stage within the item, stages of it, ring position
@@ -960,9 +974,8 @@ int launch_cfg(const TcParams &p0, int scale_dtype, const void *x, int64_t x_row
   rc = cached_map(&tw, p.wq, CU_TENSOR_MAP_DATA_TYPE_UINT32, (uint64_t)p.K / 8, (uint64_t)w_rows, (uint64_t)p.K / 2,
                   kChunkK / 8, kBN);
   if (rc != ZT_SUCCESS) return rc;
-  // Scales and zero points travel with the packed chunks (one or two groups x 128 columns per chunk) when a
-  // group is a power of two of at least 128 k and the tables can be addressed by TMA; otherwise the conversion
-  // threads fetch them from global memory.
+  // Scales and zero points travel with the packed chunks when the group size is a power of two, the tables can be
+  // addressed by TMA and a chunk's part of them fits its slot; otherwise the conversion threads fetch them from global memory.
   CUtensorMap ts = tw, tz = tw;
   p.staged_gpc = 0;
   p.groups = p.K / p.gs;
@@ -973,8 +986,9 @@ int launch_cfg(const TcParams &p0, int scale_dtype, const void *x, int64_t x_row
     const uint64_t esz = scale_dtype == ZT_F32 ? 4 : 2;
     const bool aligned = ((uint64_t)p.N * esz) % 16 == 0 && (reinterpret_cast<uintptr_t>(p.scales) & 15) == 0 &&
                          (!asym || (reinterpret_cast<uintptr_t>(p.zeros) & 15) == 0);
-    if (p.gs_log2 >= 7 && aligned) {
-      p.staged_gpc = p.gs == 128 ? 2 : 1;
+    const int gpc = p.gs >= kChunkK ? 1 : kChunkK / p.gs;
+    if (p.gs_log2 >= 0 && aligned && (size_t)gpc * kBN * esz * (asym ? 2 : 1) <= (size_t)scale_slot_bytes(NMAX)) {
+      p.staged_gpc = gpc;
       const uint64_t table_rows = (uint64_t)(w_rows / p.N) * (uint64_t)p.groups;   // experts x groups
       const CUtensorMapDataType sdt = scale_dtype == ZT_F32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
       rc = cached_map(&ts, p.scales, sdt, (uint64_t)p.N, table_rows, (uint64_t)p.N * esz, kBN, (uint32_t)p.staged_gpc, false);
