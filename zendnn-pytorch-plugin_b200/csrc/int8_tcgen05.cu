@@ -98,7 +98,7 @@ int launch_cfg(const CUtensorMap &ta, const CUtensorMap &tb, const TcParams &p, 
   if (int rc = allow_dynamic_smem(configured, kern, kSmemLimit)) return rc;
   const int tiles = p.m_tiles * p.n_tiles, sms = sm_count();
   const dim3 grid((unsigned)(tiles < sms ? tiles : sms));
-  ZT_CUDA_OK(launch_overlapped(kern, grid, dim3(kThreads), (size_t)smem_bytes(MH, p.stages, p.stage_bytes), st, ta, tb, p));
+  ZT_CUDA_OK(launch_overlapped(kern, grid, dim3(kThreads), (size_t)smem_bytes(p.stages, p.stage_bytes, p.ring_pad), st, ta, tb, p));
   return launch_status("int8_tcgen05_kernel");
 }
 template <int MH>
@@ -157,11 +157,12 @@ int int8_tcgen05_launch(const Int8GemmArgs &a, cudaStream_t st) {
   p.n_tiles = ceil_div(p.N, tile.bn);
   // A stage costs its producer two copies, an expect and a wait, about 400 cycles whatever their size; small tiles take up to
   // four 128-byte blocks of K per stage while at least four stages fit (M = 1 on 8192 -> 10240: 22.3 -> 21.2 us; M = 16 on 4096 -> 11008 with narrower boxes 19.5 -> 12.7 us).
-  const int block_bytes = (p.a_rows + tile.bn) * kBK, room = kSmemLimit - smem_bytes(tile.mh, 0, tile.mh * kBM * kBK);
+  const int block_bytes = (p.a_rows + tile.bn) * kBK, room = kSmemLimit - smem_bytes(0, 0, 0);
   p.group = 1;
   while (p.group < 4 && a.K % kBK == 0 && p.group * kBK < a.K && 2 * p.group * block_bytes * 4 <= room) p.group *= 2;
   p.stage_bytes = p.group * block_bytes;
-  p.stages = std::min(kMaxStages, (kSmemLimit - smem_bytes(tile.mh, 0, p.stage_bytes)) / p.stage_bytes);
+  p.ring_pad = ring_pad(tile.mh, p.a_rows, tile.bn, p.group);
+  p.stages = std::min(kMaxStages, (kSmemLimit - smem_bytes(0, 0, p.ring_pad)) / p.stage_bytes);
   CUtensorMap ta, tb;
   // q_rows: rows that may be addressed behind q (the caller's scratch is padded to kMinQRows rows so that the
   // activation map never has fewer; rows beyond M hold stale bytes whose products are never stored)

@@ -10,17 +10,18 @@
 // stage for two 128-row accumulators, which halves the weight bytes pulled per MAC) (tiles that share a weight column
 // block are adjacent in the order, so they run at the same time on neighbouring SMs and the weight
 // block is fetched from HBM once).  The tile's width BN is a run-time argument (pick_tile in int8_tcgen05.cu).  The
-// int32 accumulator lives in tensor memory and is double buffered up to 512 columns in all, so the epilogue of tile i overlaps the main loop of tile i+1:
+// int32 accumulator lives in tensor memory and is double buffered up to 512 columns in all, so the epilogue of tile i overlaps
+// the main loop of tile i+1:
 //
-//   warp 0      TMA producer (one lane): fills the shared-memory ring, across tile boundaries
-//   warp 1      allocates tensor memory, issues the MMAs (one lane), frees tensor memory
+//   warp 0      TMA producer: fills the shared-memory ring, across tile boundaries
+//   warp 1      allocates tensor memory, issues the MMAs, frees tensor memory
 //   warps 2..9  epilogue: tcgen05.ld the accumulator (lane == output row; two warps per 32-lane
 //               quarter, each taking every other 32-column chunk), scale, bias, post-op, cast,
 //               16-byte stores
 //
-// The roles' control flow is uniform across their warp (see tc05.cuh) and the issuer looks at the next stage's
-// barrier while it issues: M = 1 on 8192 -> 10240 25.5 -> 22.4 us; M = 512 and larger, bound by operand delivery out of L2
-// and by power, did not change.
+// The producer and the issuer run as whole warps, one lane issuing, with uniform control flow (see tc05.cuh), and the
+// issuer looks at the next stage's barrier while it issues: M = 1 on 8192 -> 10240 25.5 -> 22.4 us; M = 512 and larger, bound
+// by operand delivery out of L2 and by power, did not change.
 //
 // Ring stages are recycled through full/empty mbarriers (tcgen05.commit frees a stage when the MMAs
 // that read it retire); accumulator buffers through tmem_full/tmem_empty mbarriers.  Every wait is
@@ -51,8 +52,9 @@ struct TcParams {
   int M, N, K;
   int m_tiles, n_tiles;
   // tile and ring, chosen by the host (see pick_tile): tile width (a multiple of 16), accumulator buffers, rows of an
-  // activation box (MH * 128, or fewer when the call has fewer), ring stages, 128-byte blocks of K per stage, stage size
-  int bn, nbuf, a_rows, stages, group, stage_bytes;
+  // activation box (MH * 128, or fewer when the call has fewer), ring stages, 128-byte blocks of K per stage, stage size,
+  // bytes behind the ring that the MMAs may read
+  int bn, nbuf, a_rows, stages, group, stage_bytes, ring_pad;
   // epilogue
   const float *src_scale;  // [M]
   const int32_t *src_zp;   // [M] or null
@@ -72,17 +74,20 @@ struct TcParams {
 };
 
 // Dynamic shared memory: the ring, then the vectors and the barriers.  The MMA always reads MH * 128 rows of A; with
-// fewer in a stage it runs on into what follows (rows that are never stored), so the ring is padded to keep that inside.
+// fewer in a stage it runs on into what follows (rows that are never stored), so the ring is padded to keep that inside:
+// furthest from the last of the stage's blocks of K.
 constexpr int kVecBytes = 2 * 3 * kMaxBN * 4;            // per accumulator buffer: w_scale, bias, rowsum
 constexpr int kBarBytes = (2 * kMaxStages + 4) * 8 + 8;
 constexpr int kSmemLimit = 227 * 1024;
 // Columns of tensor memory of a 128-row accumulator.
 __host__ __device__ constexpr int acc_stride(int bn) { return (bn + 31) & ~31; }
-__host__ __device__ constexpr int ring_pad(int mh, int stage_bytes) {
-  return mh * kBM * kBK > stage_bytes ? mh * kBM * kBK - stage_bytes : 0;
+constexpr int ring_pad(int mh, int a_rows, int bn, int group) {
+  const int read = ((group - 1) * a_rows + mh * kBM) * kBK, stage_bytes = group * (a_rows + bn) * kBK;
+  return read > stage_bytes ? read - stage_bytes : 0;
 }
-__host__ __device__ constexpr int smem_bytes(int mh, int stages, int stage_bytes) {
-  return stages * stage_bytes + ring_pad(mh, stage_bytes) + kVecBytes + kBarBytes + 1024;   // + slack to align to 1024
+static_assert(ring_pad(1, 16, 16, 4) == 48 * kBK && ring_pad(1, 48, 16, 2) == 48 * kBK && ring_pad(1, 128, 16, 1) == 0, "reads past a stage");
+constexpr int smem_bytes(int stages, int stage_bytes, int pad) {
+  return stages * stage_bytes + pad + kVecBytes + kBarBytes + 1024;   // + slack to align to 1024
 }
 
 // A post-op chain on `n` (up to 32) consecutive outputs of one row.  The chain's code exists once, in a loop: unrolled over
@@ -253,7 +258,7 @@ __global__ void __launch_bounds__(kThreads, 1) int8_tcgen05_kernel(const __grid_
   unsigned char *smem = smem_dyn + ((1024u - (smem_u32(smem_dyn) & 1023u)) & 1023u);
   const int BN = p.bn, STAGES = p.stages;
   const uint32_t stage_bytes = (uint32_t)p.stage_bytes, a_bytes = (uint32_t)(p.a_rows * p.group) * kBK, NBUF = (uint32_t)p.nbuf;
-  unsigned char *after_ring = smem + STAGES * stage_bytes + ring_pad(MH, p.stage_bytes);
+  unsigned char *after_ring = smem + STAGES * stage_bytes + p.ring_pad;
   float *s_vec = reinterpret_cast<float *>(after_ring);  // [2][3][kMaxBN]
   uint64_t *full_bar = reinterpret_cast<uint64_t *>(after_ring + kVecBytes);
   uint64_t *empty_bar = full_bar + kMaxStages;
