@@ -61,6 +61,28 @@ def test_dynamic_quantize_nan_and_signed_zero(capi):
         assert (y[4] == 0).all()
 
 
+@pytest.mark.parametrize("k", [4096, 8192, 8200])
+def test_special_values_in_few_long_rows(capi, k):
+    """The same in the 1024-thread form, which few rows of at least 4096 values take: NaN in one thread's last chunk, -0, and
+    infinities (the scale is infinite; what else is finite becomes 0)."""
+    g = torch.Generator().manual_seed(k)
+    x = (torch.randn(4, k, generator=g) * 2).to(torch.bfloat16)
+    x[0, k - 3] = float("nan")
+    x[1] = -0.0
+    x[2, 5], x[2, k - 1] = float("inf"), -float("inf")
+    for act in (capi.ZT_ACT_S8_SYM, capi.ZT_ACT_U8_ASYM):
+        q, s, zp = (t.cpu() for t in capi.dynamic_quantize(x.cuda(), act))
+        if act == capi.ZT_ACT_S8_SYM:
+            q_ref, s_ref = O.dynamic_quantize_s8(x)
+            zp_ref = torch.zeros(4, dtype=torch.int32)
+            assert torch.equal(q[2, 6:k - 1], torch.zeros(k - 7, dtype=torch.int8))
+        else:
+            q_ref, s_ref, zp_ref = O.dynamic_quantize_u8(x)
+        assert torch.isnan(s[0]) and torch.isinf(s[2]) and torch.isinf(s_ref[2])
+        assert torch.equal(s[[1, 3]], s_ref[[1, 3]]) and not torch.signbit(s[1])
+        assert torch.equal(q[[1, 3]], q_ref[[1, 3]]) and torch.equal(zp[[1, 3]], zp_ref[[1, 3]])
+
+
 TILES = [0, 64, 96, 128, 160, 192, 224, 256, 1128, 1160, 1192, 1256]  # +1000: 256-row CTA tiles
 
 
