@@ -81,7 +81,17 @@ __device__ __forceinline__ bool mbar_try_addr(uint32_t addr, uint32_t parity) {
       : "memory");
   return done != 0;
 }
-// Same, for waits that are expected to last: each poll may suspend the warp for up to `hint_ns`
+// The same without suspending.
+__device__ __forceinline__ uint32_t mbar_test_addr(uint32_t addr, uint32_t parity) {
+  uint32_t done;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(done)
+      : "r"(addr), "r"(parity)
+      : "memory");
+  return done;
+}
+// mbar_wait for waits that are expected to last: each poll may suspend the warp for up to `hint_ns`
 // (it wakes when the phase completes), so a waiting warp takes almost no issue slots.
 __device__ __forceinline__ bool mbar_wait_suspend(uint64_t *bar, uint32_t parity, uint32_t sleep_ns = 100,
                                                   uint32_t hint_ns = 2000) {
@@ -134,20 +144,6 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t cols) {
 }
 __device__ __forceinline__ void fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-// Makes generic-proxy writes to shared memory visible to the async proxy (TMA / tcgen05 reads).
-__device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-
-// The same without suspending.
-__device__ __forceinline__ uint32_t mbar_test_addr(uint32_t addr, uint32_t parity) {
-  uint32_t done;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(done)
-      : "r"(addr), "r"(parity)
-      : "memory");
-  return done;
-}
-
 // ---- whole-warp roles -----------------------------------------------------------------------------
 // Index of the warp, from a shuffle: the compiler then knows that branches on it are uniform across the warp and keeps
 // what a role computes (descriptors, barrier addresses) in uniform registers.
