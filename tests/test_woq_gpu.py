@@ -239,6 +239,9 @@ def test_tcgen05_accumulation_error(capi, m, k, n, limit):
     (20, 14336, 136, 128, False, torch.float32, 32),     # two column tiles, the last eight wide
     (17, 8256, 130, 64, True, torch.bfloat16, 32),       # K = 32 x 256 + 64: slices of unequal length, the last with a void stage; odd row pitch
     (24, 2816, 640, 64, True, torch.float32, 32),        # eleven chunks; scales and zero points of four groups a chunk
+    (20, 4096, 4000, 128, False, torch.float32, 32),     # up to eight slices are a cluster: here four, 32 clusters
+    (50, 2816, 2500, 64, True, torch.bfloat16, 64),      # eleven chunks, unequal slices
+    (100, 1024, 1001, 128, False, torch.float32, 128),   # one chunk each, odd number of columns
     (50, 4416, 520, 64, False, torch.float32, 64),       # the last slice has 64 k in its last chunk
     (60, 4096, 1024, 32, True, torch.bfloat16, 64),      # eight groups a chunk
     (64, 12288, 257, 12288, True, torch.float32, 64),    # one group, odd number of columns

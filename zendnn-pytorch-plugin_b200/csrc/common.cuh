@@ -98,10 +98,10 @@ inline cudaError_t launch_overlapped(Kernel kern, dim3 grid, dim3 block, size_t 
   return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
-// The same, as thread-block clusters of `cluster` CTAs (the cluster spans the grid's y dimension).
+// The same, as thread-block clusters.
 template <typename Kernel, typename... Args>
 inline cudaError_t launch_overlapped_cluster(Kernel kern, dim3 grid, dim3 block, size_t smem, cudaStream_t st,
-                                             unsigned cluster_y, Args... args) {
+                                             dim3 cluster, Args... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -109,9 +109,9 @@ inline cudaError_t launch_overlapped_cluster(Kernel kern, dim3 grid, dim3 block,
   cfg.stream = st;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 1;
-  attr[0].val.clusterDim.y = cluster_y;
-  attr[0].val.clusterDim.z = 1;
+  attr[0].val.clusterDim.x = cluster.x;
+  attr[0].val.clusterDim.y = cluster.y;
+  attr[0].val.clusterDim.z = cluster.z;
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;

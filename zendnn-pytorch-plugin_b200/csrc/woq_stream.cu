@@ -403,7 +403,7 @@ int launch(const StreamParams &p_in, dim3 grid, cudaStream_t st) {
   p.early_trigger = (long long)grid.x * grid.y * 2 <= (long long)per_sm * sm_count() ? 1 : 0;
   if (cluster) {
     // a cluster shape the device cannot place is refused at launch: fall back to the reduction through the workspace
-    if (launch_overlapped_cluster(kern, grid, dim3(S::W * 32), smem, st, (unsigned)p.nsplit, p) == cudaSuccess)
+    if (launch_overlapped_cluster(kern, grid, dim3(S::W * 32), smem, st, dim3(1, (unsigned)p.nsplit), p) == cudaSuccess)
       return launch_status("woq_stream_kernel");
     (void)cudaGetLastError();
     cluster = false;

@@ -38,10 +38,10 @@
 // are requested long before use because a copy takes over a thousand cycles), packed chunks of 256 k.
 //
 // Work split.  An item is a tile, or a slice of its K (whole chunks) where there are fewer tiles than SMs or a shorter sum is
-// wanted (see min_sums and dense_plan); the slices' fp32 sums go through the workspace and a second kernel adds them in order,
-// so results do not depend on timing.  Without slices the layers of few tiles leave most SMs idle: M = 17 on 4096 -> 4096 took
-// 12.8 us on 32 SMs and takes 7.9 in four slices.  The slices used to meet at the end of this kernel by tickets, which cost 5 - 10
-// us and so was hardly ever worth it.
+// wanted (see min_sums and dense_plan).  The slices' fp32 sums are added in order, so results do not depend on timing: by a
+// cluster through its shared memory, or by a second kernel through the workspace (see launch_cfg).  Without slices the layers
+// of few tiles leave most SMs idle: M = 17 on 4096 -> 4096 took 12.8 us on 32 SMs and takes 7.9 in four slices.  The slices used to
+// meet at the end of this kernel by tickets, which cost 5 - 10 us and so was hardly ever worth it.
 //
 // Sums.  The tensor core's fp32 accumulation truncates, so its error grows with the length of the sum: tiles of up to 128 rows
 // are therefore summed in two accumulators, one for each parity of the 64-k blocks, which the epilogue adds.
@@ -58,6 +58,7 @@
 // (both bf16) and dq = fma(q, s_hi, q*s_lo), which equals bf16(q*s) except for rare double-rounding cases one bf16
 // ulp apart; the zero-point form is evaluated in fp32 and rounded once.
 #include <algorithm>
+#include <atomic>
 #include <mutex>
 #include <unordered_map>
 
@@ -80,6 +81,7 @@ constexpr int kChunkBytes = kBN * 128;
 // the activation ring leaves no room for that, tables that need more than 4 KB are read from global memory)
 __host__ __device__ constexpr int scale_slot_bytes(int nmax) { return nmax == 64 ? 4096 : 8192; }
 constexpr int kMaxSlices = 32;      // K slices of a tile
+constexpr int kMaxCluster = 8;      // of them added by a cluster (the portable size)
 
 // How a weight is dequantised (template parameter of the kernel).
 enum DqMode { kSymF32 = 0, kSymBf16 = 1, kAsymBf16 = 2, kAsymF32 = 3 };
@@ -99,7 +101,8 @@ struct TcParams {
   __nv_bfloat16 *y;
   PostOpsDev post;
   int *status;
-  float *partial;             // slices > 1: their sums [slices][M][N rounded up to 4], which woq_slices_kernel adds
+  int cluster;                // slices > 1: a tile's slices are a cluster, which adds them through shared memory ...
+  float *partial;             // ... or else their sums [slices][M][N rounded up to 4], which woq_slices_kernel adds
   // grouped mode (g_count != nullptr)
   const int *g_count;         // number of row tiles
   const int4 *g_tiles;        // per row tile: {expert, first row, valid rows, 0}
@@ -173,6 +176,7 @@ struct SmemLayout {
   static constexpr int kPackedBytes = PSTAGES * kChunkBytes;
   static constexpr int kScaleBytes = PSTAGES * scale_slot_bytes(NMAX);
   static constexpr int kBarBytes = (2 * SLOTS + 2 * XSTAGES + 2 * PSTAGES + 5) * 8 + 8;
+  static_assert(NMAX * kBN * 4 <= kXRing, "sums of a slice");
   static constexpr int kTotal = kXRing + kPackedBytes + kScaleBytes + kBarBytes + 1024;
 };
 
@@ -778,21 +782,42 @@ __global__ void __launch_bounds__(threads_for(TEAMS), 1) woq_tcgen05_kernel(cons
       }
     };
     const bool with_operands = p.post.bufs[0] != nullptr && !p.partial;
-    const int jobs = (ti.rows + 15) >> 4, stride = last ? TEAMS + 1 : 1, job0 = last ? (int)group : 0;
-    if (with_operands && job0 < jobs) request(job0);
+    const int jobs = (ti.rows + 15) >> 4;
+    int stride = last ? TEAMS + 1 : 1, job0 = last ? (int)group : 0;
+    // the jobs that this warp finishes: of a cluster's every CTA takes its share
+    const int end_stride = p.cluster ? stride * p.slices : stride, end_job0 = p.cluster ? job0 * p.slices + (int)wd.slice : job0;
+    if (with_operands && end_job0 < jobs) request(end_job0);
     ok = ok && tc::warp_wait_idle(last ? smem_u32(last_full) : smem_u32(&tmem_full[acc.set]), last ? 0u : (acc.use & 1));
     if (!ok && lane == 0) tc::report_timeout(p.status, kStatusEpilogueTimeout);
     tc::fence_after_sync();
     const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc.col;
     // the second accumulator, unless the item has only 64 k (a tail of K)
     const bool add_second = two && min(p.K, (int)wd.c1 * kChunkK) - (int)wd.c0 * kChunkK > 64;
+    const uint32_t sums = smem_u32(smem) + (uint32_t)(quarter * 32 + lane) * 4;   // cluster: [tokens][128], over the activation ring
+    // A cluster first leaves its slices' sums in shared memory, then adds them in order.
+#pragma unroll 1
+    for (bool add = false;; add = true) {
+    if (add) {
+      tc::cluster_sync();
+      job0 = end_job0;
+      stride = end_stride;
+    }
 #pragma unroll 1
     for (int job = job0; job < jobs; job += stride) {
       // rows past the valid ones belong to nobody, or to the next expert
       const int rows = live ? min(16, ti.rows - job * 16) : 0;
       const int64_t row0 = ti.m0 + job * 16, at = row0 * p.N + n;
       float v[16];
-      {
+      if (add) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] = 0.f;
+#pragma unroll 2
+        for (int s = 0; s < p.slices; ++s) {
+          const uint32_t src = tc::map_to_rank(sums, (uint32_t)s) + (uint32_t)job * (16 * kBN * 4);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) v[j] += tc::load_cluster_f32(src + j * (kBN * 4));
+        }
+      } else {
         uint32_t r[16];
         tc::tmem_ld_32x32b_x16(t_row + job * 16, r);
         if (add_second) {
@@ -811,6 +836,12 @@ __global__ void __launch_bounds__(threads_for(TEAMS), 1) woq_tcgen05_kernel(cons
         tc::fence_before_sync();
         __syncwarp();
         tc::arrive_if(lane == 0, smem_u32(&tmem_empty[acc.set]));
+      }
+      if (p.cluster && !add) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+          asm volatile("st.shared.f32 [%0], %1;" ::"r"(sums + (uint32_t)(job * 16 + j) * (kBN * 4)), "f"(v[j]) : "memory");
+        continue;
       }
       if (p.partial) {                                   // the sums of this slice; bias and post-ops come when they are added
         const int64_t pitch = (p.N + 3) & ~3;
@@ -846,7 +877,13 @@ __global__ void __launch_bounds__(threads_for(TEAMS), 1) woq_tcgen05_kernel(cons
         if (j < rows) *dst = __float2bfloat16_rn(v[j]);
       if (with_operands && job + stride < jobs) request(job + stride);
     }
+    if (add || !p.cluster) break;
+    }
   }
+  }
+  if (p.cluster) {
+    if (warp < 3) tc::cluster_sync();      // the other warps' first
+    tc::cluster_sync();                    // a peer may still read this CTA's sums
   }
 
   tc::fence_before_sync();
@@ -957,9 +994,38 @@ int cached_map(CUtensorMap *out, const void *ptr, CUtensorMapDataType dt, uint64
   return ZT_SUCCESS;
 }
 
+// How many clusters of a size the device can run at once, asked for once per device and size.
+struct ClusterRoom {
+  std::atomic<int> known[64][kMaxCluster + 1] = {};   // + 1
+  template <typename Kernel>
+  int clusters(Kernel kern, int threads, int smem, int size) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+    std::atomic<int> &entry = known[dev][size];
+    if (const int k = entry.load(std::memory_order_relaxed)) return k - 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)size);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = (unsigned)size;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      n = 0;
+    }
+    entry.store(n + 1, std::memory_order_relaxed);
+    return n;
+  }
+};
+
 template <int NMAX, int KS, int TEAMS, int SLOTS, int XK, int XSTAGES, int PSTAGES>
 int launch_cfg(const TcParams &p0, int scale_dtype, const void *x, int64_t x_rows, int64_t w_rows, int max_row_tiles,
-               cudaStream_t st) {
+               bool *slices_added, cudaStream_t st) {
   using L = SmemLayout<NMAX, KS, TEAMS, SLOTS, XK, XSTAGES, PSTAGES>;
   static_assert(L::kTotal <= 227 * 1024, "rings exceed shared memory");
   TcParams p = p0;
@@ -1006,6 +1072,22 @@ int launch_cfg(const TcParams &p0, int scale_dtype, const void *x, int64_t x_row
   static PerDeviceOnce configured[4];
   auto launch = [&](auto kern, int which) -> int {
     if (int rc_cfg = allow_dynamic_smem(configured[which], kern, L::kTotal)) return rc_cfg;
+    // Slices are added by clusters where there are two of them (M = 128, 8192 -> 8192: 22.3 us with the second kernel, 19.7
+    // so), and where a slice is so short that submitting a second kernel takes longer than the call (M = 100, 1024 -> 1024 called
+    // in a row: 10.2 and 7.5 us, although on the device it is 6.2 and 7.2).  Larger clusters of longer slices start later than as
+    // many single CTAs: M = 17, 4096 -> 4096 in four slices 7.9 us with the second kernel and 10.1 as clusters.
+    static ClusterRoom room[4];
+    const bool cluster = p.slices == 2 || (p.slices > 2 && p.slices <= kMaxCluster && p.chunks <= 2 * p.slices);
+    if (cluster && items <= sms &&
+        room[which].clusters(kern, threads_for(TEAMS), L::kTotal, p.slices) * p.slices >= items) {
+      TcParams c = p;
+      c.cluster = 1;
+      c.partial = nullptr;
+      *slices_added = true;
+      ZT_CUDA_OK(launch_overlapped_cluster(kern, grid, dim3(threads_for(TEAMS)), (size_t)L::kTotal, st, dim3((unsigned)p.slices), tx, tx2,
+                                           tw, ts, tz, c));
+      return launch_status("woq_tcgen05_kernel");
+    }
     ZT_CUDA_OK(launch_overlapped(kern, grid, dim3(threads_for(TEAMS)), (size_t)L::kTotal, st, tx, tx2, tw, ts, tz, p));
     return launch_status("woq_tcgen05_kernel");
   };
@@ -1018,13 +1100,13 @@ int launch_cfg(const TcParams &p0, int scale_dtype, const void *x, int64_t x_row
 
 // `cap`: the instantiation's largest token tile
 int launch_any(int cap, const TcParams &p, int scale_dtype, const void *x, int64_t x_rows, int64_t w_rows,
-               int max_row_tiles, cudaStream_t st) {
+               int max_row_tiles, bool *slices_added, cudaStream_t st) {
   switch (cap) {
     // <token tile, k per stage, conversion teams, converted slots, k per activation slot, activation slots, packed chunks>
-    case 32: return launch_cfg<32, 128, 6, 6, 256, 5, 6>(p, scale_dtype, x, x_rows, w_rows, max_row_tiles, st);
-    case 64: return launch_cfg<64, 128, 6, 6, 256, 3, 6>(p, scale_dtype, x, x_rows, w_rows, max_row_tiles, st);
-    case 128: return launch_cfg<128, 128, 4, 4, 128, 4, 4>(p, scale_dtype, x, x_rows, w_rows, max_row_tiles, st);
-    case 192: return launch_cfg<192, 64, 4, 4, 64, 5, 4>(p, scale_dtype, x, x_rows, w_rows, max_row_tiles, st);
+    case 32: return launch_cfg<32, 128, 6, 6, 256, 5, 6>(p, scale_dtype, x, x_rows, w_rows, max_row_tiles, slices_added, st);
+    case 64: return launch_cfg<64, 128, 6, 6, 256, 3, 6>(p, scale_dtype, x, x_rows, w_rows, max_row_tiles, slices_added, st);
+    case 128: return launch_cfg<128, 128, 4, 4, 128, 4, 4>(p, scale_dtype, x, x_rows, w_rows, max_row_tiles, slices_added, st);
+    case 192: return launch_cfg<192, 64, 4, 4, 64, 5, 4>(p, scale_dtype, x, x_rows, w_rows, max_row_tiles, slices_added, st);
     default: break;
   }
   set_error("zt_woq_linear: unsupported token-tile width %d for the tcgen05 kernel", cap);
@@ -1144,8 +1226,9 @@ int woq_tcgen05_launch(const zt_woq_linear_args_t &a, cudaStream_t st) {
   p.accs = d.accs;
   p.x_box = p.x_box2 = d.m_tiles == 1 ? (int)ceil_div<int64_t>(a.M, 8) * 8 : d.bt;   // 128-byte swizzle: 8-row atoms
   p.partial = d.slices > 1 ? reinterpret_cast<float *>(reinterpret_cast<char *>(a.workspace) + ZT_WOQ_COUNTER_BYTES) : nullptr;
-  const int rc = launch_any(d.cap, p, a.scale_dtype, a.x, a.M, a.N, 0, st);
-  if (rc != ZT_SUCCESS || d.slices == 1) return rc;
+  bool slices_added = d.slices == 1;
+  const int rc = launch_any(d.cap, p, a.scale_dtype, a.x, a.M, a.N, 0, &slices_added, st);
+  if (rc != ZT_SUCCESS || slices_added) return rc;
   const int64_t quads = a.M * ceil_div<int64_t>(a.N, 4);
   ZT_CUDA_OK(launch_overlapped(woq_slices_kernel, dim3((unsigned)ceil_div<int64_t>(quads, kSliceThreads)), dim3(kSliceThreads), (size_t)0, st,
                                (const float *)p.partial, d.slices, p.M, p.N, p.bias, p.bias_dtype, p.post, p.y));
@@ -1176,7 +1259,8 @@ int woq_tcgen05_grouped_launch(const void *x, int64_t total_rows, int64_t N, int
   p.x_box2 = row_tile;
   p.g_count = tile_count;
   p.g_tiles = tiles;
-  return launch_any(cap_for(row_tile), p, scale_dtype, x, total_rows, (int64_t)num_experts * N, max_row_tiles, st);
+  bool slices_added = true;
+  return launch_any(cap_for(row_tile), p, scale_dtype, x, total_rows, (int64_t)num_experts * N, max_row_tiles, &slices_added, st);
 }
 
 }  // namespace zt
