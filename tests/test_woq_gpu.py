@@ -272,6 +272,17 @@ def test_tcgen05_k_slices(capi, m, k, n, gs, asym, scale_dtype, cap):
     assert_close_bf16(ym, O.woq_linear(x, packed.t(), s, z, b, ops, bufs), what=f"K slices, mul_add {m}x{k}x{n}")
 
 
+@pytest.mark.parametrize("m,k,n", [(20, 4096, 4000), (20, 14336, 136)])
+def test_tcgen05_no_room_for_slices(capi, monkeypatch, m, k, n):
+    """A workspace that does not hold the slices' sums: all of K by one CTA, in two accumulators."""
+    x, q, s, _, b = make_woq_case(m, k, n, 128, seed=m)
+    y, packed = _run(capi, x, q, s, None, b, capi.ZT_ALGO_TCGEN05)
+    monkeypatch.setattr(capi, "woq_workspace", lambda nbytes, device: torch.zeros(capi.ZT_WOQ_COUNTER_BYTES, dtype=torch.uint8, device=device))
+    whole, _ = _run(capi, x, q, s, None, b, capi.ZT_ALGO_TCGEN05)
+    assert_close_bf16(whole, O.woq_linear(x, packed.t(), s, None, b), what=f"no room for slices {m}x{k}x{n}")
+    assert not torch.equal(y, whole)
+
+
 @pytest.mark.parametrize("name", sorted(["relu", "gelu_erf", "silu", "add", "mul_add", "add_add"]))
 def test_tcgen05_post_ops(capi, name):
     ops, nbuf = POST_CASES[name]

@@ -92,7 +92,9 @@ constexpr int smem_bytes(int stages, int stage_bytes, int pad) {
 
 // A post-op chain on `n` (up to 32) consecutive outputs of one row.  The chain's code exists once, in a loop: unrolled over
 // the 32 values (and its four steps) it is some hundred kilobytes of instructions that a tile walks through once, which
-// made a 384 x 4096 x 1024 call of the static form take 55 us with 3 % of the issue slots used (13.8 us now).
+// made a 384 x 4096 x 1024 call of the static form take 54 us with 3 % of the issue slots used (12.2 us without a chain now,
+// 30 with an addition and 52 with a multiplication and an addition, where it took 75 and 108; the dynamic form on 512 x 4096
+// x 4096 37 and 58 us for 84 and 118).
 __device__ __forceinline__ void post_chain(float (&v)[32], const PostOpsDev &post, int64_t base, int n, int dtype) {
   float w[32];          // indexed by the loop, so it lives in local memory; `v` stays in registers
 #pragma unroll
