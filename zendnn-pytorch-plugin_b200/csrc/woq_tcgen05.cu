@@ -20,7 +20,7 @@
 // of eight weights 9 shift / permute / lop3 operations on one and 8 - 12 bf16x2 operations on the other); its MMAs take 2
 // cycles per token and at least 128.  A block takes 300 - 350 cycles up to 64 tokens and 350 - 450 up to 128 (650 when the
 // converted operand went through shared memory and the issuing threads ran divergent code); per call, M = 32 on 4096 -> 14336:
-// 21.6 -> 15.0 us, M = 128 on 8192 -> 8192 with two operands: 39.4 -> 25.6 us, M = 2048 on 4096 -> 14336: 263 -> 219 us (0.66 of the
+// 21.6 -> 14.8 us, M = 128 on 8192 -> 8192 with two operands: 39.4 -> 24.9 us, M = 2048 on 4096 -> 14336: 263 -> 217 us (0.67 of the
 // bf16 peak; from 128 tokens on an SM pulls 35 bytes per cycle of activations and weights out of L2, which is what it can
 // get).  What that took:
 //   * The converted operand lives in tensor memory: its 32 KB per block (store, then MMA read) leave the shared-memory
@@ -782,75 +782,11 @@ __global__ void __launch_bounds__(threads_for(TEAMS), 1) woq_tcgen05_kernel(cons
       }
     };
     const bool with_operands = p.post.bufs[0] != nullptr && !p.partial;
-    const int jobs = (ti.rows + 15) >> 4;
-    int stride = last ? TEAMS + 1 : 1, job0 = last ? (int)group : 0;
-    // the jobs that this warp finishes: of a cluster's every CTA takes its share
-    const int end_stride = p.cluster ? stride * p.slices : stride, end_job0 = p.cluster ? job0 * p.slices + (int)wd.slice : job0;
-    if (with_operands && end_job0 < jobs) request(end_job0);
-    ok = ok && tc::warp_wait_idle(last ? smem_u32(last_full) : smem_u32(&tmem_full[acc.set]), last ? 0u : (acc.use & 1));
-    if (!ok && lane == 0) tc::report_timeout(p.status, kStatusEpilogueTimeout);
-    tc::fence_after_sync();
-    const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc.col;
-    // the second accumulator, unless the item has only 64 k (a tail of K)
-    const bool add_second = two && min(p.K, (int)wd.c1 * kChunkK) - (int)wd.c0 * kChunkK > 64;
-    const uint32_t sums = smem_u32(smem) + (uint32_t)(quarter * 32 + lane) * 4;   // cluster: [tokens][128], over the activation ring
-    // A cluster first leaves its slices' sums in shared memory, then adds them in order.
-#pragma unroll 1
-    for (bool add = false;; add = true) {
-    if (add) {
-      tc::cluster_sync();
-      job0 = end_job0;
-      stride = end_stride;
-    }
-#pragma unroll 1
-    for (int job = job0; job < jobs; job += stride) {
+    // bias, post-ops and store of a job's sums
+    auto finish = [&](int job, float (&v)[16]) {
       // rows past the valid ones belong to nobody, or to the next expert
       const int rows = live ? min(16, ti.rows - job * 16) : 0;
-      const int64_t row0 = ti.m0 + job * 16, at = row0 * p.N + n;
-      float v[16];
-      if (add) {
-#pragma unroll
-        for (int j = 0; j < 16; ++j) v[j] = 0.f;
-#pragma unroll 2
-        for (int s = 0; s < p.slices; ++s) {
-          const uint32_t src = tc::map_to_rank(sums, (uint32_t)s) + (uint32_t)job * (16 * kBN * 4);
-#pragma unroll
-          for (int j = 0; j < 16; ++j) v[j] += tc::load_cluster_f32(src + j * (kBN * 4));
-        }
-      } else {
-        uint32_t r[16];
-        tc::tmem_ld_32x32b_x16(t_row + job * 16, r);
-        if (add_second) {
-          uint32_t r2[16];
-          tc::tmem_ld_32x32b_x16(t_row + acc.second + job * 16, r2);
-          tc::tmem_ld_wait();
-#pragma unroll
-          for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]) + __uint_as_float(r2[j]);
-        } else {
-          tc::tmem_ld_wait();
-#pragma unroll
-          for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
-        }
-      }
-      if (!last && job + stride >= jobs) {               // read: the next tile may be summed here
-        tc::fence_before_sync();
-        __syncwarp();
-        tc::arrive_if(lane == 0, smem_u32(&tmem_empty[acc.set]));
-      }
-      if (p.cluster && !add) {
-#pragma unroll
-        for (int j = 0; j < 16; ++j)
-          asm volatile("st.shared.f32 [%0], %1;" ::"r"(sums + (uint32_t)(job * 16 + j) * (kBN * 4)), "f"(v[j]) : "memory");
-        continue;
-      }
-      if (p.partial) {                                   // the sums of this slice; bias and post-ops come when they are added
-        const int64_t pitch = (p.N + 3) & ~3;
-        float *dst = p.partial + ((int64_t)wd.slice * p.M + row0) * pitch + n;
-#pragma unroll
-        for (int j = 0; j < 16; ++j, dst += pitch)
-          if (j < rows) __stcg(dst, v[j]);
-        continue;
-      }
+      const int64_t at = (int64_t)(ti.m0 + job * 16) * p.N + n;
 #pragma unroll
       for (int j = 0; j < 16; ++j) v[j] += bias;
       int b = 0;
@@ -875,9 +811,73 @@ __global__ void __launch_bounds__(threads_for(TEAMS), 1) woq_tcgen05_kernel(cons
 #pragma unroll
       for (int j = 0; j < 16; ++j, dst += p.N)
         if (j < rows) *dst = __float2bfloat16_rn(v[j]);
-      if (with_operands && job + stride < jobs) request(job + stride);
+    };
+    const int jobs = (ti.rows + 15) >> 4, stride = last ? TEAMS + 1 : 1, job0 = last ? (int)group : 0;
+    // of a cluster's jobs every CTA finishes its share
+    const int first = p.cluster ? job0 * p.slices + (int)wd.slice : job0;
+    if (with_operands && first < jobs) request(first);
+    ok = ok && tc::warp_wait_idle(last ? smem_u32(last_full) : smem_u32(&tmem_full[acc.set]), last ? 0u : (acc.use & 1));
+    if (!ok && lane == 0) tc::report_timeout(p.status, kStatusEpilogueTimeout);
+    tc::fence_after_sync();
+    const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc.col;
+    // the second accumulator, unless the item has only 64 k (a tail of K)
+    const bool add_second = two && min(p.K, (int)wd.c1 * kChunkK) - (int)wd.c0 * kChunkK > 64;
+    const uint32_t sums = smem_u32(smem) + (uint32_t)(quarter * 32 + lane) * 4;   // cluster: [tokens][128], over the activation ring
+#pragma unroll 1
+    for (int job = job0; job < jobs; job += stride) {
+      float v[16];
+      {
+        uint32_t r[16];
+        tc::tmem_ld_32x32b_x16(t_row + job * 16, r);
+        if (add_second) {
+          uint32_t r2[16];
+          tc::tmem_ld_32x32b_x16(t_row + acc.second + job * 16, r2);
+          tc::tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]) + __uint_as_float(r2[j]);
+        } else {
+          tc::tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
+        }
+      }
+      if (!last && job + stride >= jobs) {               // read: the next tile may be summed here
+        tc::fence_before_sync();
+        __syncwarp();
+        tc::arrive_if(lane == 0, smem_u32(&tmem_empty[acc.set]));
+      }
+      if (p.slices == 1) {
+        finish(job, v);
+        if (with_operands && job + stride < jobs) request(job + stride);
+      } else if (p.cluster) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+          asm volatile("st.shared.f32 [%0], %1;" ::"r"(sums + (uint32_t)(job * 16 + j) * (kBN * 4)), "f"(v[j]) : "memory");
+      } else {                                           // the sums of this slice; bias and post-ops come when they are added
+        const int rows = live ? min(16, ti.rows - job * 16) : 0;
+        const int64_t pitch = (p.N + 3) & ~3;
+        float *dst = p.partial + ((int64_t)wd.slice * p.M + ti.m0 + job * 16) * pitch + n;
+#pragma unroll
+        for (int j = 0; j < 16; ++j, dst += pitch)
+          if (j < rows) __stcg(dst, v[j]);
+      }
     }
-    if (add || !p.cluster) break;
+    if (p.cluster) {                                     // all slices' sums are in shared memory: add them in order
+      tc::cluster_sync();
+#pragma unroll 1
+      for (int job = first; job < jobs; job += stride * p.slices) {
+        float v[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] = 0.f;
+#pragma unroll 2
+        for (int s = 0; s < p.slices; ++s) {
+          const uint32_t src = tc::map_to_rank(sums, (uint32_t)s) + (uint32_t)job * (16 * kBN * 4);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) v[j] += tc::load_cluster_f32(src + j * (kBN * 4));
+        }
+        finish(job, v);
+        if (with_operands && job + stride * p.slices < jobs) request(job + stride * p.slices);
+      }
     }
   }
   }
