@@ -1137,8 +1137,8 @@ int64_t min_sums(int64_t M, int64_t N, int64_t K) {
 // The number of row tiles and of K slices by estimated cycles.  A 128 x 64 block takes the slower of the conversion
 // (350 cycles, 400 where it calculates in fp32) and the MMAs (2 per token, and about 90 around them), and then waits for its
 // operands out of L2 the longer, the more rows a tile has and the more SMs pull; adding slices up takes a launch of its own
-// (5000 cycles) and their way through L2.  The constants are fitted to 108 shapes of 130 - 1024 rows timed with every plan:
-// the chosen one is 1 % above the fastest in the mean and 11 % at most.  M = 192, 14336 -> 4096: 53 us in one slice, 22.5 in
+// (5000 cycles; the same is charged where a cluster does it) and their way through L2.  The constants are fitted to 108 shapes of 130 - 1024 rows timed with every plan:
+// the chosen one is 0.7 % above the fastest in the mean and 9 % at most.  M = 192, 14336 -> 4096: 53 us in one slice, 22.5 in
 // four; M = 384: 39 as 2 x 2, 53 as three row tiles of whole K; M = 256, 2816 -> 5003: 14.0 whole, 21.6 in two slices.
 DensePlan dense_plan(int64_t M, int64_t N, int64_t K, bool fp32_conversion, bool may_slice) {
   const int64_t sms = sm_count(), n_tiles = ceil_div<int64_t>(N, kBN), chunks = ceil_div<int64_t>(K, kChunkK);
